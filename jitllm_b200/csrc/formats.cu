@@ -120,6 +120,20 @@ __global__ void repack_mxfp4_kernel(const uint8_t *__restrict__ raw, uint8_t *__
     }
 }
 
+// raw [rows][k/256] x 210 B  ->  ql, qh, sc [rows][k/256][208], d [rows][k/256]. One thread per 16-byte word of the result
+// (13 a block), the last of a block also moves d.
+__global__ void repack_q6_k_kernel(const uint8_t *__restrict__ raw, uint8_t *__restrict__ blocks, uint16_t *__restrict__ d, size_t nblk) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nblk * 13; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t b = i / 13;
+        const int c = (int)(i - b * 13);
+        const uint16_t *src = reinterpret_cast<const uint16_t *>(raw + b * 210 + c * 16);
+        uint32_t w[4];
+        for (int j = 0; j < 4; j++) w[j] = (uint32_t)src[2 * j] | ((uint32_t)src[2 * j + 1] << 16);
+        *reinterpret_cast<uint4 *>(blocks + b * JL_Q6K_BLOCK + c * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (c == 12) d[b] = src[8];
+    }
+}
+
 void jl_weight_release(jl_weight *w) {
     if (!w) return;
     if (w->zc_exec) cudaGraphExecDestroy((cudaGraphExec_t)w->zc_exec);
@@ -158,7 +172,7 @@ int jl_repack_upload(jl_ctx *ctx, uint32_t type, const void *w_host, size_t w_by
         if (w->emin > w->emax) { w->emin = 127; w->emax = 127; }
     }
     cudaError_t e;
-    if (type == JL_TYPE_Q4_K || jl_type_raw_simt(type)) {
+    if (type == JL_TYPE_Q4_K || (jl_type_raw_simt(type) && type != JL_TYPE_Q6_K)) {
         // +16 so a kernel may over-read one aligned chunk past the end.
         w->data_bytes = need;
         if ((e = cudaMalloc(&w->data, need + 16)) != cudaSuccess) goto oom;
@@ -181,6 +195,14 @@ int jl_repack_upload(jl_ctx *ctx, uint32_t type, const void *w_host, size_t w_by
             if ((e = cudaMalloc(&w->data, w->data_bytes + 16)) != cudaSuccess) { cudaFree(raw); goto oom; }
             if ((e = cudaMalloc(&w->scales, w->scales_bytes + 16)) != cudaSuccess) { cudaFree(raw); goto oom; }
             repack_q8_0_kernel<<<grid, 256, 0, ctx->stream>>>(raw, w->data, (uint16_t *)w->scales, rows, k);
+        } else if (type == JL_TYPE_Q6_K) {
+            const size_t nb6 = rows * (size_t)(k / 256);
+            w->data_bytes = nb6 * JL_Q6K_BLOCK;
+            w->scale_stride = k / 256;
+            w->scales_bytes = nb6 * 2;
+            if ((e = cudaMalloc(&w->data, w->data_bytes + 16)) != cudaSuccess) { cudaFree(raw); goto oom; }
+            if ((e = cudaMalloc(&w->scales, w->scales_bytes + 16)) != cudaSuccess) { cudaFree(raw); goto oom; }
+            repack_q6_k_kernel<<<148 * 8, 256, 0, ctx->stream>>>(raw, w->data, (uint16_t *)w->scales, nb6);
         } else {
             w->data_bytes = nblk * 16;
             w->scale_stride = ((k / 32) + 15) / 16 * 16;
@@ -239,13 +261,18 @@ __global__ void unpack_resident_kernel(uint32_t type, const uint8_t *__restrict_
             for (int l = 0; l < 32; l++) q[r * 32 + l] = (int8_t)((s & 1) ? (grp[l] >> 4) : (grp[l] & 0xF));
         } else if (jl_type_raw_simt(type)) {
             // raw blocks: sub-block si of the row (Q6_K: two 16-element records)
-            const int be = jl_block_elems(type), bb = jl_block_bytes(type);
-            const uint8_t *blk = data + (row * (size_t)(k / be) + (size_t)(si * 32 / be)) * bb;
+            const int be = jl_block_elems(type), bb = type == JL_TYPE_Q6_K ? JL_Q6K_BLOCK : jl_block_bytes(type);
+            const size_t b = row * (size_t)(k / be) + (size_t)(si * 32 / be);
+            const uint8_t *blk = data + b * bb;
             const int e0 = (si * 32) % be;
             for (int l = 0; l < 32; l++) q[r * 32 + l] = (int8_t)jl_raw_code(type, blk, e0 + l);
             if (type == JL_TYPE_Q6_K) {
-                jl_raw_record(type, blk, e0 / 16, &d_bits[2 * r], &dmin_bits[2 * r], &sc[2 * r], &m[2 * r]);
-                jl_raw_record(type, blk, e0 / 16 + 1, &d_bits[2 * r + 1], &dmin_bits[2 * r + 1], &sc[2 * r + 1], &m[2 * r + 1]);
+                for (int h = 0; h < 2; h++) {              // d lives in the scales plane
+                    d_bits[2 * r + h] = ((const uint16_t *)scales)[b];
+                    dmin_bits[2 * r + h] = 0;
+                    sc[2 * r + h] = (uint8_t)((int)(int8_t)blk[192 + e0 / 16 + h] + 128);
+                    m[2 * r + h] = 0;
+                }
             } else {
                 jl_raw_record(type, blk, e0 / 32, &d_bits[r], &dmin_bits[r], &sc[r], &m[r]);
             }

@@ -118,61 +118,105 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const uint8_t *__restric
     if (lane == 0) Y[(size_t)tok * nrows + row] = acc;
 }
 
-// Q6_K decode without a byte loop: one warp per row, two super-blocks per pass. A super-block is two halves of 128
-// elements; in a half, byte l of ql / ql + 32 / qh carries elements l, l + 32, l + 64, l + 96 (low nibbles, low
-// nibbles of the second run, high nibbles, high nibbles; two bits of qh each). Eight lanes take a half, lane i of them
-// the four positions l = 4i .. 4i + 3: three 32-bit words (read as 16-bit halves: a 210-byte block is only 2-byte
-// aligned) give it 16 codes, which become floats by byte placement (0x4B0000qq reads as 2^23 + q), and its four
-// float4 of the activation row. Each weight is formed as quant.Dequant32 forms it: (d * sc) rounded, times (q - 32)
-// rounded (format/quant/dequant.go:443-470). NT tokens share the decoded weights.
-__device__ __forceinline__ uint32_t q6k_ld32(const uint8_t *p) {
-    const uint16_t *h = reinterpret_cast<const uint16_t *>(p);
-    return (uint32_t)__ldg(h) | ((uint32_t)__ldg(h + 1) << 16);
+// Q6_K decode: a block of threads takes R rows, a thread of it one unit (half n, 16-run j) of a super-block at a time --
+// a quarter of it, 64 codes: three 16-byte words of codes, eight scale bytes and d per row, and the 64 activations that go
+// with them, loaded once for the R rows. A super-block is two halves of 128 elements; in a half, byte l of ql / ql + 32 /
+// qh carries elements l, l + 32, l + 64, l + 96 (low nibbles, low nibbles of the second run, high nibbles, high nibbles;
+// two bits of qh each), so 16 consecutive l are four runs of 16 consecutive elements, each with a scale of its own.
+// Codes become floats by byte placement (0x4B0000qq reads as 2^23 + q; minus (2^23 + 32) = q - 32, exact); a run's sum of
+// (q - 32) x is weighted by d * sc, which f32 holds exactly, so no weight is rounded at all. NT tokens share the codes.
+// Bound by what is in flight: a lane that read 2-byte words of the 210-byte blocks took 38.0 us for one token of 4096 x 14336;
+// the resident 208-byte blocks (see jl_weight) are read in 16-byte words, R x 58 bytes a thread at a time: 19.8 us, 2.4 TB/s.
+__device__ __forceinline__ void q6k_fma2(float2 &acc, float2 a, float2 b) {
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\t"
+        "mov.b64 ra, {%2, %3};\n\t"
+        "mov.b64 rb, {%4, %5};\n\t"
+        "mov.b64 rc, {%0, %1};\n\t"
+        "fma.rn.f32x2 rc, ra, rb, rc;\n\t"
+        "mov.b64 {%0, %1}, rc;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
 }
-template <int NT>
-__global__ void __launch_bounds__(256) gemv_q6k_kernel(const uint8_t *__restrict__ data, const float *__restrict__ X,
-                                                       float *__restrict__ Y, int nrows, int k, int ntok) {
-    const int row = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    const int tok0 = blockIdx.y * NT;
-    if (row >= nrows) return;
+template <int R, int NT>
+__global__ void __launch_bounds__(256) gemv_q6k_kernel(const uint8_t *__restrict__ data, const uint16_t *__restrict__ dplane,
+                                                       const float *__restrict__ X, float *__restrict__ Y, int nrows, int k, int ntok) {
+    __shared__ float red[8][R * NT];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row0 = blockIdx.x * R, tok0 = blockIdx.y * NT;
     const int nsb = k / 256;
-    const int hl = lane >> 3, i = lane & 7;            // half hl of the pass's two super-blocks, positions 4i..4i+3
-    const int n = hl & 1;
-    const uint8_t *rowp = data + (size_t)row * nsb * 210;
-    float acc[NT];
+    float acc[R][NT];
 #pragma unroll
-    for (int t = 0; t < NT; t++) acc[t] = 0.f;
-    for (int sb = hl >> 1; sb < nsb; sb += 2) {
-        const uint8_t *blk = rowp + (size_t)sb * 210;
-        const uint32_t A = q6k_ld32(blk + n * 64 + 4 * i), B = q6k_ld32(blk + n * 64 + 32 + 4 * i);
-        const uint32_t H = q6k_ld32(blk + 128 + n * 32 + 4 * i);
-        const float d = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const uint16_t *>(blk + 208))));
-        const int8_t *scp = reinterpret_cast<const int8_t *>(blk + 192 + n * 8 + (i >> 2));
-        // the four 32-runs of the half: codes of positions 4i..4i+3, one byte each
-        const uint32_t c4[4] = {(A & 0x0F0F0F0Fu) | ((H & 0x03030303u) << 4), (B & 0x0F0F0F0Fu) | ((H & 0x0C0C0C0Cu) << 2),
-                                ((A >> 4) & 0x0F0F0F0Fu) | (H & 0x30303030u), ((B >> 4) & 0x0F0F0F0Fu) | ((H & 0xC0C0C0C0u) >> 2)};
+    for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const float dsc = __fmul_rn(d, (float)(int)__ldg(scp + 2 * c));
-            float w[4];
+        for (int t = 0; t < NT; t++) acc[r][t] = 0.f;
+    for (int u = tid; u < nsb * 4; u += blockDim.x) {
+        const int sb = u >> 2, n = (u >> 1) & 1, j = u & 1;
+        uint4 A[R], B[R], H[R];
+        uint2 S[R];
+        float d[R];
 #pragma unroll
-            for (int j = 0; j < 4; j++)   // 0x4B0000qq = 2^23 + q; minus (2^23 + 32) = q - 32, exact
-                w[j] = __fmul_rn(dsc, __uint_as_float(__byte_perm(c4[c], 0x4B000000u, 0x7650 + j)) - 8388640.f);
-            const size_t e0 = (size_t)sb * 256 + n * 128 + c * 32 + 4 * i;
+        for (int r = 0; r < R; r++) {
+            const size_t b = (size_t)min(row0 + r, nrows - 1) * nsb + sb;      // rows past the end repeat the last
+            const uint8_t *blk = data + b * JL_Q6K_BLOCK;
+            A[r] = ldg16(blk + n * 64 + 16 * j);
+            B[r] = ldg16(blk + n * 64 + 32 + 16 * j);
+            H[r] = ldg16(blk + 128 + n * 32 + 16 * j);
+            S[r] = __ldg(reinterpret_cast<const uint2 *>(blk + 192 + n * 8));
+            d[r] = half_bits_to_float(__ldg(dplane + b));
+        }
+        const float *xu = X + (size_t)tok0 * k + (size_t)sb * 256 + n * 128 + j * 16;
 #pragma unroll
-            for (int t = 0; t < NT; t++) {
-                if (tok0 + t < ntok) {
-                    const float4 x = __ldg(reinterpret_cast<const float4 *>(X + (size_t)(tok0 + t) * k + e0));
-                    acc[t] = fmaf(w[0], x.x, acc[t]); acc[t] = fmaf(w[1], x.y, acc[t]);
-                    acc[t] = fmaf(w[2], x.z, acc[t]); acc[t] = fmaf(w[3], x.w, acc[t]);
+        for (int c = 0; c < 4; c++) {                  // the run of elements c * 32 + 16 j .. + 15 of the half
+            float2 g[R][NT];
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int t = 0; t < NT; t++) g[r][t] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                float4 x[NT];
+#pragma unroll
+                for (int t = 0; t < NT; t++)
+                    x[t] = tok0 + t < ntok ? __ldg(reinterpret_cast<const float4 *>(xu + (size_t)t * k + c * 32) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const uint4 L = (c & 1) ? B[r] : A[r];
+                    const uint32_t l = i == 0 ? L.x : i == 1 ? L.y : i == 2 ? L.z : L.w;
+                    const uint32_t h = i == 0 ? H[r].x : i == 1 ? H[r].y : i == 2 ? H[r].z : H[r].w;
+                    const uint32_t hb = c == 0 ? h << 4 : c == 1 ? h << 2 : c == 2 ? h : h >> 2;
+                    const uint32_t q4 = ((c < 2 ? l : l >> 4) & 0x0F0F0F0Fu) | (hb & 0x30303030u);
+                    float w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) w[e] = __uint_as_float(__byte_perm(q4, 0x4B000000u, 0x7650 + e)) - 8388640.f;
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        q6k_fma2(g[r][t], make_float2(w[0], w[1]), make_float2(x[t].x, x[t].y));
+                        q6k_fma2(g[r][t], make_float2(w[2], w[3]), make_float2(x[t].z, x[t].w));
+                    }
                 }
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int sc = (int)(int8_t)((c < 2 ? S[r].x : S[r].y) >> (16 * (c & 1) + 8 * j));   // scale byte j + 2c
+                const float dsc = d[r] * (float)sc;
+#pragma unroll
+                for (int t = 0; t < NT; t++) acc[r][t] = fmaf(g[r][t].x + g[r][t].y, dsc, acc[r][t]);
             }
         }
     }
 #pragma unroll
-    for (int t = 0; t < NT; t++) {
-        const float v = warp_sum(acc[t]);
-        if (lane == 0 && tok0 + t < ntok) Y[(size_t)(tok0 + t) * nrows + row] = v;
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            const float v = warp_sum(acc[r][t]);
+            if (lane == 0) red[warp][r * NT + t] = v;
+        }
+    __syncthreads();
+    if (tid < R * NT) {
+        float v = red[0][tid];
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) v += red[w][tid];   // fixed order
+        const int r = tid / NT, t = tid % NT;
+        if (row0 + r < nrows && tok0 + t < ntok) Y[(size_t)(tok0 + t) * nrows + row0 + r] = v;
     }
 }
 
@@ -684,6 +728,10 @@ int jl_gemv_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, jl_ch
         c.kernel = JL_K_SIMT; c.warps = 8; c.rows_per_cta = 8; c.split_k = 1;
         c.grid = (nrows + 7) / 8 * ntok;
         c.launches = 1;
+        if (type == JL_TYPE_Q6_K) {                    // a block of threads per 4 rows (one token) or per 2 rows x 4 tokens
+            c.warps = min(8, (k / 64 + 31) / 32); c.rows_per_cta = ntok == 1 ? 4 : 2; c.split_k = 1;
+            c.grid = (nrows + c.rows_per_cta - 1) / c.rows_per_cta * (ntok == 1 ? 1 : (ntok + 3) / 4);
+        }
     } else {
         const int idx = q4k_pick(ctx, nrows, k / 256, ntok, true);
         if (idx < 0) return JL_DECLINED;
@@ -699,7 +747,8 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
     size_t rows_off = (size_t)expert * nrows;
     const uint8_t *data = w->data;
     const uint8_t *scales = w->scales;
-    if (w->type == JL_TYPE_Q4_K || jl_type_raw_simt(w->type)) data += rows_off * jl_row_bytes(w->type, k);
+    if (w->type == JL_TYPE_Q6_K) { data += rows_off * (size_t)(k / 256) * JL_Q6K_BLOCK; scales += rows_off * (size_t)w->scale_stride * 2; }
+    else if (w->type == JL_TYPE_Q4_K || jl_type_raw_simt(w->type)) data += rows_off * jl_row_bytes(w->type, k);
     else if (w->type == JL_TYPE_Q8_0) { data += rows_off * (size_t)k; scales += rows_off * (size_t)w->scale_stride * 2; }
     else { data += rows_off * (size_t)(k / 32) * 16; scales += rows_off * (size_t)w->scale_stride; }
 
@@ -752,7 +801,12 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
 #define JL_ROWK45(T) do { if (ntok == 1) gemv_q45_kernel<T, 1><<<g1, 256, 0, s>>>(data, x_dev, out_dev, nrows, k, ntok); \
                            else gemv_q45_kernel<T, 4><<<g4, 256, 0, s>>>(data, x_dev, out_dev, nrows, k, ntok); } while (0)
         // the raw formats' own row kernels (a lane takes many codes at a time; up to four tokens share the decoded weights)
-        if (w->type == JL_TYPE_Q6_K) JL_ROWK(gemv_q6k_kernel);
+        if (w->type == JL_TYPE_Q6_K) {
+            const uint16_t *d = reinterpret_cast<const uint16_t *>(scales);
+            const int threads = min(256, (k / 64 + 31) / 32 * 32);            // a thread per unit of the row, up to 256
+            if (ntok == 1) gemv_q6k_kernel<4, 1><<<dim3((nrows + 3) / 4, 1), threads, 0, s>>>(data, d, x_dev, out_dev, nrows, k, ntok);
+            else gemv_q6k_kernel<2, 4><<<dim3((nrows + 1) / 2, (ntok + 3) / 4), threads, 0, s>>>(data, d, x_dev, out_dev, nrows, k, ntok);
+        }
         else if (w->type == JL_TYPE_Q5_K) JL_ROWK(gemv_q5k_kernel);
         else if (w->type == JL_TYPE_Q4_0) JL_ROWK45(JL_TYPE_Q4_0);
         else if (w->type == JL_TYPE_Q5_0) JL_ROWK45(JL_TYPE_Q5_0);
@@ -766,7 +820,7 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
         else if (w->type == JL_TYPE_MXFP4)
             gemv_simt_kernel<JL_TYPE_MXFP4><<<grid, 256, 0, s>>>(data, scales, w->scale_stride, x_dev, out_dev, nrows, k, ntok);
 #define JL_SIMT_RAW(T) else if (w->type == T) gemv_simt_kernel<T><<<grid, 256, 0, s>>>(data, scales, w->scale_stride, x_dev, out_dev, nrows, k, ntok);
-        JL_SIMT_RAW(JL_TYPE_Q4_0) JL_SIMT_RAW(JL_TYPE_Q5_0) JL_SIMT_RAW(JL_TYPE_Q5_1) JL_SIMT_RAW(JL_TYPE_Q5_K) JL_SIMT_RAW(JL_TYPE_Q6_K)
+        JL_SIMT_RAW(JL_TYPE_Q4_0) JL_SIMT_RAW(JL_TYPE_Q5_0) JL_SIMT_RAW(JL_TYPE_Q5_1) JL_SIMT_RAW(JL_TYPE_Q5_K)
 #undef JL_SIMT_RAW
         else return jl_set_err(ctx, JL_DECLINED, "type %u has no decode kernel", w->type);
     }

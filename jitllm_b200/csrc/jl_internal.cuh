@@ -41,7 +41,7 @@ __host__ __device__ static inline int jl_block_bytes(uint32_t t) {
     }
     return 0;
 }
-// Formats that stay as raw ggml blocks on the device and run on the one-warp-per-row kernel only.
+// Formats without an integer tensor-core decode kernel: row kernels over (nearly) raw blocks.
 __host__ __device__ static inline bool jl_type_raw_simt(uint32_t t) {
     return t == JL_TYPE_Q4_0 || t == JL_TYPE_Q5_0 || t == JL_TYPE_Q5_1 || t == JL_TYPE_Q5_K || t == JL_TYPE_Q6_K;
 }
@@ -64,7 +64,10 @@ static inline size_t jl_row_bytes(uint32_t t, int k) {
 //          which one mma.sync lane consumes them. scales = f16 d, [row][k/32].
 //   MXFP4  data = the 16 code bytes of each block, [row][k/32][16];
 //          scales = the e8m0 byte of each block, [row][scale_stride].
-//   Q4_0, Q5_0, Q5_1, Q5_K, Q6_K   data = the raw blocks, untouched.
+//   Q6_K   data = the first 208 bytes of each block (ql, qh, sc), [row][k/256][208]: 13 aligned 16-byte words where the
+//          raw 210-byte blocks are only 2-byte aligned; scales = the f16 d of each block, [row][k/256].
+//   Q4_0, Q5_0, Q5_1, Q5_K   data = the raw blocks, untouched.
+#define JL_Q6K_BLOCK 208
 struct jl_weight {
     uint32_t type;
     int n_expert, nrows, k;
