@@ -59,6 +59,8 @@ JL_EXPORT int jl_open(int device, const jl_opts *opts, jl_ctx **out) {
     c->dev_status = nullptr;
     c->stat_pin = nullptr;
     c->moe_stage = nullptr; c->moe_stage_cap = 0;
+    c->q6k_work = nullptr; c->q6k_cap = 0; c->reserved_k = c->reserved_tok = c->q6k_k = 0;
+    c->q6k_stream = nullptr; c->q6k_done = nullptr; c->q6k_recorded = false;
     c->x_map = c->o_map = nullptr; c->x_map_cap = c->o_map_cap = 0; c->done_map = nullptr; c->done_seq = 0;
     const int words[4] = {0, (int)c->opts.wait_limit_us, 0, 0};   // code, wait limit, the done kernel's sequence counter, spare
     if (cudaMalloc(&c->dev_status, sizeof words) != cudaSuccess ||
@@ -90,6 +92,8 @@ JL_EXPORT void jl_close(jl_ctx *ctx) {
     if (ctx->x_dev) cudaFree(ctx->x_dev);
     if (ctx->o_dev) cudaFree(ctx->o_dev);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->q6k_work) cudaFree(ctx->q6k_work);
+    if (ctx->q6k_done) cudaEventDestroy(ctx->q6k_done);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->x_pin) cudaFreeHost(ctx->x_pin);
     if (ctx->o_pin) cudaFreeHost(ctx->o_pin);
@@ -186,6 +190,9 @@ JL_EXPORT int jl_reserve(jl_ctx *ctx, int max_rows, int max_k, int max_tok) {
     if (max_tok > 8 && need_gemm > need) need = need_gemm;
     int rc = jl_grow_scratch(ctx, need);
     if (rc) return rc;
+    if (k256 > ctx->reserved_k) ctx->reserved_k = k256;
+    if (max_tok > ctx->reserved_tok) ctx->reserved_tok = max_tok;
+    if (ctx->q6k_k && (rc = jl_gemm_q6k_reserve(ctx, ctx->q6k_k > ctx->reserved_k ? ctx->reserved_k : ctx->q6k_k, ctx->reserved_tok))) return rc;
     return reserve_locked(ctx, (size_t)max_tok * max_k * 4, (size_t)max_tok * max_rows * 4);
 }
 
@@ -342,6 +349,10 @@ JL_EXPORT int jl_weight_upload_bank(jl_ctx *ctx, uint32_t type, const void *w_ho
     int rc = jl_grow_scratch(ctx, jl_gemv_scratch_bytes(type, k, type == JL_TYPE_Q8_0 ? 32 : 8));
     if (rc) return rc;
     rc = jl_repack_upload(ctx, type, w_host, w_bytes, n_expert, nrows, k, out);
+    if (rc == JL_OK && type == JL_TYPE_Q6_K) {     // the batch kernel's workspace, for as many tokens as were reserved
+        if (k > ctx->q6k_k) ctx->q6k_k = k;
+        if ((rc = jl_gemm_q6k_reserve(ctx, ctx->q6k_k, ctx->reserved_tok))) { jl_weight_release(*out); *out = nullptr; return rc; }
+    }
     if (rc == JL_OK) {
         std::lock_guard<std::mutex> lk2(ctx->cache_mu);
         ctx->st.resident_bytes += (*out)->raw_bytes;
@@ -378,6 +389,9 @@ static int choose(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, jl_cho
     if ((pin == JL_K_TC5 || (pin == JL_K_AUTO && ntok > decode_max)) && jl_gemm_tc5_supported(type, nrows, k, ntok))
         return jl_gemm_tc5_choice(ctx, type, nrows, k, ntok, out);
     if (pin == JL_K_TC5) return JL_DECLINED;
+    // Q6_K above 8 tokens: the integer GEMM, when its workspace is there (up to 8 the row kernel decodes a weight for
+    // four tokens at a time and needs no prepared activations)
+    if (type == JL_TYPE_Q6_K && ntok > 8 && jl_gemm_q6k_choice(ctx, nrows, k, ntok, out) == JL_OK) return JL_OK;
     return jl_gemv_choice(ctx, type, nrows, k, ntok, out);
 }
 
@@ -397,7 +411,7 @@ static int matmul_dev_locked(jl_ctx *ctx, void *out_dev, int out_dtype, const jl
     jl_choice ch;
     int rc = choose(ctx, w->type, w->nrows, w->k, ntok, &ch);
     if (rc) return rc == JL_DECLINED ? jl_set_err(ctx, JL_DECLINED, "pinned kernel cannot serve this shape") : rc;
-    if (ch.kernel == JL_K_TC5)
+    if (ch.kernel == JL_K_TC5 && w->type != JL_TYPE_Q6_K)
         return jl_launch_gemm_tc5(ctx, out_dev, out_dtype, w, expert, x_dev, x_dtype, ntok, s);
     if (x_dtype != JL_DT_F32 || out_dtype != JL_DT_F32) {
         // 16-bit activations or outputs: the GEMM converts them, the decode kernels do not
@@ -405,6 +419,7 @@ static int matmul_dev_locked(jl_ctx *ctx, void *out_dev, int out_dtype, const jl
             return jl_launch_gemm_tc5(ctx, out_dev, out_dtype, w, expert, x_dev, x_dtype, ntok, s);
         return jl_set_err(ctx, JL_DECLINED, "the decode kernels take f32 activations and outputs");
     }
+    if (ch.kernel == JL_K_TC5) return jl_launch_gemm_q6k(ctx, (float *)out_dev, w, expert, (const float *)x_dev, ntok, s);
     return jl_launch_gemv(ctx, (float *)out_dev, w, expert, (const float *)x_dev, ntok, ch.kernel, s);
 }
 
@@ -562,6 +577,7 @@ static int matmul_host(jl_ctx *ctx, void *out, int out_dtype, uint32_t type, con
         const size_t need_gemm = jl_gemm_tc5_scratch_bytes(nrows, k, ntok, x_dtype, ctx->sm_count);
         if (need_gemm > need) need = need_gemm;
         if ((rc = jl_grow_scratch(ctx, need))) return rc;
+        if (type == JL_TYPE_Q6_K && (rc = jl_gemm_q6k_reserve(ctx, k, ntok))) return rc;
     }
     {
         // Decode calls (a few tokens, f32 in and out): no copy engine and no stream synchronisation on the path. The

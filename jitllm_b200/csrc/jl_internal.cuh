@@ -115,6 +115,11 @@ struct jl_ctx {
     void *x_dev; size_t x_cap;
     void *o_dev; size_t o_cap;
     void *scratch; size_t scratch_cap;
+    // workspace of the Q6_K batch kernel, apart from the scratch (whose prepared operands outlive a call): sized for
+    // what jl_reserve and the Q6_K uploads have asked for. q6k_done orders calls that come on another stream.
+    void *q6k_work; size_t q6k_cap;
+    int reserved_k, reserved_tok, q6k_k;
+    cudaStream_t q6k_stream; cudaEvent_t q6k_done; bool q6k_recorded;
     void *x_pin; size_t x_pin_cap;
     void *o_pin; size_t o_pin_cap;
     int *dev_status;        // device words: [0] code a kernel sets when a bounded wait ran out, [1] the limit (us)
@@ -179,6 +184,12 @@ int jl_matmul_keyed(jl_ctx *ctx, void *out, int out_dtype, uint32_t type, const 
                     const void *x, int x_dtype, int nrows, int k, int ntok);
 void jl_drain_graveyard(jl_ctx *ctx);
 int jl_read_status(jl_ctx *ctx, cudaStream_t s);
+
+// gemm_q6k.cu -- Q6_K for 9 tokens and more (tcgen05, integer). f32 in and out.
+size_t jl_gemm_q6k_scratch_bytes(int k, int ntok);
+int jl_gemm_q6k_choice(jl_ctx *ctx, int nrows, int k, int ntok, jl_choice *out);
+int jl_gemm_q6k_reserve(jl_ctx *ctx, int k, int ntok);
+int jl_launch_gemm_q6k(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, const float *x_dev, int ntok, cudaStream_t s);
 
 // gemm_tc5.cu -- prefill kernels (tcgen05).
 int jl_gemm_tc5_operand(jl_ctx *ctx, const jl_weight *w, int ntok, void **rows, float **inv_scale);

@@ -1,9 +1,9 @@
-"""Q6_K on the row kernel."""
+"""Q6_K: the integer GEMM that serves 9 tokens and more, and the row kernel below."""
 import numpy as np
 import pytest
 import torch
 
-from jitllm_b200 import K_SIMT, Q6_K, Device, synth
+from jitllm_b200 import K_SIMT, K_TC5, Q6_K, Device, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -23,6 +23,59 @@ def run(dev, w, nrows, k, x):
     assert dev.lib.jl_status_poll(dev.ctx, None) == 0
     h.free()
     return out.cpu().numpy()
+
+
+# one super-block and one row, tile edges (128 rows; 16, 32, 64 tokens), every number of k slices, odd rows and tokens
+@pytest.mark.parametrize("nrows,k,ntok", [(1, 256, 9), (37, 512, 16), (128, 768, 17), (129, 1024, 32), (300, 2048, 33), (256, 1280, 64),
+                                          (511, 3584, 65), (4096, 4096, 203), (16384, 512, 64), (1024, 14336, 130)])
+def test_batch_kernel_matches_float64(orc, nrows, k, ntok):
+    rng = synth.rng_for(0xB600 + nrows + k + ntok)
+    w, x = synth.matrix(rng, Q6_K, nrows, k), synth.activations(rng, ntok, k)
+    ref = orc.matmul_f64(Q6_K, w, x, nrows, k, ntok)
+    with Device(0) as dev:
+        dev.Reserve(nrows, k, ntok)
+        h = dev.Upload(Q6_K, w, nrows, k)
+        assert dev.Select(Q6_K, nrows, k, ntok).kernel == K_TC5
+        h.free()
+        got = run(dev, w, nrows, k, x)
+        assert np.array_equal(got, run(dev, w, nrows, k, x))             # fixed order
+    # a super-block's sum is exact; joining and scaling it rounds four times, then one addition per super-block and slice
+    assert rel(got, ref) <= (4 + k / 256 / 2) * 2.0 ** -24
+    with Device(0, pin_kernel=K_SIMT) as dev:
+        simt = rel(run(dev, w, nrows, k, x), ref)
+    print(f"{nrows}x{k} {ntok} tokens: batch kernel {rel(got, ref):.2e}, row kernel {simt:.2e}")
+
+
+@pytest.mark.parametrize("dist", ["one_huge", "tiny", "huge", "zeros"])
+def test_batch_kernel_input_distributions(orc, dist):
+    rng = synth.rng_for(78)
+    nrows, k, ntok = 64, 2048, 24
+    x = rng.standard_normal((ntok, k))
+    if dist == "one_huge":
+        x[:, ::32] *= 1000.0
+    x *= dict(tiny=1e-9, huge=1e9, zeros=0.0).get(dist, 1.0)
+    x = x.astype(np.float32)
+    w = synth.matrix(rng, Q6_K, nrows, k)
+    with Device(0) as dev:
+        got = run(dev, w, nrows, k, x)
+    ref = orc.matmul_f64(Q6_K, w, x, nrows, k, ntok)
+    assert np.array_equal(got, ref) if dist == "zeros" else rel(got, ref) <= (4 + k / 256 / 2) * 2.0 ** -24
+
+
+def test_batch_kernel_not_finite():
+    """Infinities and NaN give what the row kernel gives, in their own token only."""
+    rng = synth.rng_for(79)
+    nrows, k, ntok = 130, 1024, 20
+    x = synth.activations(rng, ntok, k)
+    x[3, 5], x[7, 700], x[11, 9], x[11, 900] = np.inf, np.nan, -np.inf, 1.0
+    w = synth.matrix(rng, Q6_K, nrows, k)
+    with Device(0) as dev:
+        got = run(dev, w, nrows, k, x)
+    with Device(0, pin_kernel=K_SIMT) as dev:
+        ref = run(dev, w, nrows, k, x)
+    assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isinf(got), np.isinf(ref))
+    fin = np.isfinite(ref)
+    assert np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)]) and rel(got[fin], ref[fin]) <= 1e-6
 
 
 @pytest.mark.parametrize("nrows,k,ntok", [(1, 256, 1), (5, 512, 1), (3, 256, 2), (1023, 3328, 1), (4096, 14336, 1), (257, 768, 5), (64, 4352, 8), (70, 512, 30)])
