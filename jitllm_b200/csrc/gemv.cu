@@ -546,6 +546,172 @@ static size_t q4k_tma_smem(int warps, int stages, int nsb, bool fused = false, b
            (size_t)warps * 16 * 4 + (size_t)(warps * stages + 1) * 8;
 }
 
+// 2..8 tokens: the same tiles, operand and arithmetic, with the tokens inside the task. One warp-task's tile is read from the
+// ring and its codes and scales are unpacked once; every token then costs its eight MMAs, nine operand loads and the fold
+// (about 45 instructions against the tile's 60). With a CTA per token (the single-token kernel on a grid of tokens) each
+// token fetched and unpacked every tile again: 31 us for 5 tokens of 14336 x 4096, 6.2 a token. The operand
+// (640 B per super-block and token: 287 KB for 8 tokens of k = 14336) passes through a shared-memory ring of its own, four
+// super-blocks of all tokens a stage, filled by a warp that does nothing else; the four warps of a row group take one
+// super-block of a stage each. (Read from global memory through L1 instead, a task's loads came back one token after the
+// other: 22 us for that shape, and 61 against 42 for 8 tokens of 4096 x 14336; as it is 17.8 and 28.7, and a decode step of 8
+// sequences over two Llama-8B-wide blocks 287 us instead of 489.) RG row groups share the stage: two where the rows
+// fill the GPU with such CTAs (half the operand traffic), else one.
+#define Q4KM_WPR 4
+template <int NT, int RG>
+struct q4km_smem {
+    static constexpr int WARPS = Q4KM_WPR * RG, STAGES = 3, XS = NT <= 4 ? 3 : 2;
+    static constexpr int X_BYTES = Q4KM_WPR * NT * Q4K_XP_SB_BYTES;
+    static constexpr int X_OFS = WARPS * STAGES * Q4K_TILE_BYTES;
+    static constexpr int RED_OFS = X_OFS + XS * X_BYTES;
+    static constexpr int BAR_OFS = RED_OFS + WARPS * NT * 16 * 4;     // tile barriers [WARPS][STAGES], xfull[XS], xempty[XS]
+    static constexpr int TOTAL = BAR_OFS + (WARPS * STAGES + 2 * XS) * 8;
+};
+template <int NT, int RG>
+__global__ void __launch_bounds__((Q4KM_WPR * RG + 1) * 32, RG == 1 ? 3 : 2)
+gemv_q4k_multi_kernel(const __grid_constant__ CUtensorMap wmap, int row0, const uint8_t *__restrict__ xop, float *__restrict__ Y, int nrows,
+                      int nsb, int *status) {
+    using L = q4km_smem<NT, RG>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t bars = smem_u32(smem) + L::BAR_OFS, xfull = bars + L::WARPS * L::STAGES * 8, xempty = xfull + L::XS * 8;
+    const int rounds = (nsb + Q4KM_WPR - 1) / Q4KM_WPR;
+    const int wq = warp % Q4KM_WPR, rg = blockIdx.x * RG + warp / Q4KM_WPR;
+    const uint32_t tiles = smem_u32(smem) + warp * L::STAGES * Q4K_TILE_BYTES, tbar = bars + warp * L::STAGES * 8;
+    if (warp < L::WARPS && lane == 0) {              // the weight ring and its barriers are private to the warp: requested at once
+#pragma unroll
+        for (int s = 0; s < L::STAGES; s++) mbar_init(tbar + 8 * s, 1);
+        mbar_init_fence();
+#pragma unroll
+        for (int s = 0; s < L::STAGES; s++) {
+            const int sbi = wq + s * Q4KM_WPR;
+            if (sbi < nsb) {
+                mbar_arrive_expect_tx(tbar + 8 * s, Q4K_TILE_BYTES);
+                tma_load_2d(tiles + s * Q4K_TILE_BYTES, &wmap, sbi * 144, row0 + rg * 16, tbar + 8 * s);
+            }
+        }
+    } else if (warp == L::WARPS && lane == 0) {
+#pragma unroll
+        for (int s = 0; s < L::XS; s++) { mbar_init(xfull + 8 * s, 1); mbar_init(xempty + 8 * s, L::WARPS); }
+        mbar_init_fence();
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float acc[NT][2];
+#pragma unroll
+    for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = 0.f;
+    bool lost = false;
+    if (warp == L::WARPS) {
+        if (lane == 0) {
+            for (int i = 0; i < rounds; i++) {
+                const int s = i % L::XS;
+                if (i >= L::XS && !mbar_wait(xempty + 8 * s, ((uint32_t)(i / L::XS) & 1u) ^ 1u, status)) { lost = true; break; }
+                const uint32_t bytes = (uint32_t)min(Q4KM_WPR, nsb - i * Q4KM_WPR) * Q4K_XP_SB_BYTES;
+                mbar_arrive_expect_tx(xfull + 8 * s, bytes * NT);
+#pragma unroll
+                for (int j = 0; j < NT; j++)
+                    bulk_load_1d(smem_u32(smem) + L::X_OFS + s * L::X_BYTES + j * Q4KM_WPR * Q4K_XP_SB_BYTES,
+                                 xop + ((size_t)j * nsb + i * Q4KM_WPR) * Q4K_XP_SB_BYTES, bytes, xfull + 8 * s);
+            }
+        }
+    } else {
+        const bool bsel = ((g >> 1) == t);  // lanes that feed a non-zero B column: digit (g & 1) of group t
+        const int sh = 8 * (2 * (t & 1));
+        for (int it = 0; it < rounds; it++) {
+            const int s = it % L::STAGES, xs = it % L::XS, sb = it * Q4KM_WPR + wq;
+            if (sb < nsb) {
+                if (!__all_sync(0xffffffffu, mbar_wait(tbar + 8 * s, (uint32_t)(it / L::STAGES) & 1u, status))) { lost = true; break; }
+                const uint8_t *tile = smem + warp * L::STAGES * Q4K_TILE_BYTES + s * Q4K_TILE_BYTES;
+                const uint4 hA = *reinterpret_cast<const uint4 *>(tile + g * 144), hB = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144);
+                const uint4 qA0 = *reinterpret_cast<const uint4 *>(tile + g * 144 + 16 + 32 * t);
+                const uint4 qA1 = *reinterpret_cast<const uint4 *>(tile + g * 144 + 32 + 32 * t);
+                const uint4 qB0 = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144 + 16 + 32 * t);
+                const uint4 qB1 = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144 + 32 + 32 * t);
+                __syncwarp();  // every lane holds its share: the stage may be refilled
+                if (lane == 0) {
+                    const int nx = sb + L::STAGES * Q4KM_WPR;
+                    if (nx < nsb) {
+                        mbar_arrive_expect_tx(tbar + 8 * s, Q4K_TILE_BYTES);
+                        tma_load_2d(tiles + s * Q4K_TILE_BYTES, &wmap, nx * 144, row0 + rg * 16, tbar + 8 * s);
+                    }
+                }
+                const uint32_t wa[8] = {qA0.x, qA0.y, qA0.z, qA0.w, qA1.x, qA1.y, qA1.z, qA1.w};
+                const uint32_t wb[8] = {qB0.x, qB0.y, qB0.z, qB0.w, qB1.x, qB1.y, qB1.z, qB1.w};
+                uint32_t scp[2], mp[2];
+                float2 dd[2];
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const uint4 &h = r ? hB : hA;
+                    const uint32_t a = h.y >> sh, b = h.z >> sh, c = h.w >> sh;
+                    if (t < 2) { scp[r] = a & 0x3F3Fu; mp[r] = b & 0x3F3Fu; }
+                    else { scp[r] = (c & 0x0F0Fu) | ((a >> 2) & 0x3030u); mp[r] = ((c >> 4) & 0x0F0Fu) | ((b >> 2) & 0x3030u); }
+                    dd[r] = __half22float2(*reinterpret_cast<const __half2 *>(&h.x));
+                }
+                if (!__all_sync(0xffffffffu, mbar_wait(xfull + 8 * xs, (uint32_t)(it / L::XS) & 1u, status))) { lost = true; break; }
+                const uint8_t *xst = smem + L::X_OFS + xs * L::X_BYTES + wq * Q4K_XP_SB_BYTES;
+                const uint32_t m4 = 0x0F0F0F0Fu, h4 = 0xF0F0F0F0u;
+#pragma unroll
+                for (int j = 0; j < NT; j++) {
+                    const uint8_t *xsb = xst + j * Q4KM_WPR * Q4K_XP_SB_BYTES;
+                    const uint8_t *xf = xsb + t * Q4K_XP_GROUP_BYTES + (g & 1) * 8;
+                    const int4 ax = *reinterpret_cast<const int4 *>(xsb + Q4K_XP_AUX_OFS + t * 16);
+                    int ce[4] = {0, 0, 0, 0}, co[4] = {0, 0, 0, 0};
+#pragma unroll
+                    for (int cp = 0; cp < 4; cp++) {
+                        const uint2 fe = bsel ? *reinterpret_cast<const uint2 *>(xf + cp * 16) : make_uint2(0u, 0u);
+                        const uint2 fo = bsel ? *reinterpret_cast<const uint2 *>(xf + 64 + cp * 16) : make_uint2(0u, 0u);
+                        const uint32_t a0 = wa[2 * cp], a2 = wa[2 * cp + 1], a1 = wb[2 * cp], a3 = wb[2 * cp + 1];
+                        mma_u8s8(ce, a0 & m4, a1 & m4, a2 & m4, a3 & m4, fe.x, fe.y);
+                        mma_u8s8(co, a0 & h4, a1 & h4, a2 & h4, a3 & h4, fo.x, fo.y);
+                    }
+                    const float inv_scale = __int_as_float(ax.z);
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        const int pe = (ce[2 * r] << 8) + ce[2 * r + 1];
+                        const int po = ((co[2 * r] << 8) + co[2 * r + 1]) >> 4;
+                        const int dotq = (int)(scp[r] & 0xFF) * pe + (int)(scp[r] >> 8) * po;
+                        const int dotm = (int)(mp[r] & 0xFF) * ax.x + (int)(mp[r] >> 8) * ax.y;
+                        acc[j][r] += (dd[r].x * (float)dotq - dd[r].y * (float)dotm) * inv_scale;
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(xempty + 8 * xs);
+        }
+    }
+    if (lost && lane == 0) atomicExch(status, 1);
+    float *red = reinterpret_cast<float *>(smem + L::RED_OFS);        // [WARPS][NT][16]
+    if (warp < L::WARPS) {
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float v = acc[j][r];
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (t == 0) red[(warp * NT + j) * 16 + g + 8 * r] = v;
+            }
+    }
+    __syncthreads();
+    for (int i = tid; i < RG * NT * 16; i += (L::WARPS + 1) * 32) {
+        const int r = i & 15, j = (i >> 4) % NT, grp = i / (16 * NT), row = (blockIdx.x * RG + grp) * 16 + r;
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < Q4KM_WPR; w++) sum += red[((grp * Q4KM_WPR + w) * NT + j) * 16 + r];     // fixed order
+        if (row < nrows) Y[(size_t)j * nrows + row] = sum;
+    }
+}
+typedef void (*q4k_multi_fn)(const CUtensorMap, int, const uint8_t *, float *, int, int, int *);
+struct q4k_multi_form { q4k_multi_fn fn; int smem; };
+#define Q4K_MULTI(RG) {{nullptr, 0}, {nullptr, 0}, {gemv_q4k_multi_kernel<2, RG>, q4km_smem<2, RG>::TOTAL}, {gemv_q4k_multi_kernel<3, RG>, q4km_smem<3, RG>::TOTAL}, \
+                       {gemv_q4k_multi_kernel<4, RG>, q4km_smem<4, RG>::TOTAL}, {gemv_q4k_multi_kernel<5, RG>, q4km_smem<5, RG>::TOTAL}, \
+                       {gemv_q4k_multi_kernel<6, RG>, q4km_smem<6, RG>::TOTAL}, {gemv_q4k_multi_kernel<7, RG>, q4km_smem<7, RG>::TOTAL}, \
+                       {gemv_q4k_multi_kernel<8, RG>, q4km_smem<8, RG>::TOTAL}}
+static const q4k_multi_form q4k_multi[2][9] = {Q4K_MULTI(1), Q4K_MULTI(2)};
+// Row groups of a CTA: two once 2 x 148 such CTAs have rows (one: 444 fit).
+static int q4k_multi_rg(int nrows) { return nrows >= 32 * 296 ? 2 : 1; }
+
 // Scratch the Q4_K tensor-core decode needs for a shape (the prepared activation operand).
 size_t jl_gemv_scratch_bytes(uint32_t type, int k, int ntok) {
     if (type == JL_TYPE_Q8_0 && k % 256 == 0) return jl_gemv_q8_scratch_bytes(k, ntok);
@@ -682,6 +848,21 @@ static bool q4k_mma_ok(uint32_t type, int k) {
     return type == JL_TYPE_Q4_K && k % 256 == 0 && q4k_find(JL_FORM_SPLIT, 0, 0, 0, 0, k / 256) >= 0;
 }
 
+// 2..8 tokens go through the kernel that keeps the tokens inside the task, unless the caller pinned a form or the warps, a
+// trial or a verdict names a variant, or overlapped matvecs want one launch each.
+static bool q4k_use_multi(const jl_ctx *ctx, int nrows, int nsb, int ntok, bool have_x) {
+    const jl_opts &o = ctx->opts;
+    if (ntok < 2 || ntok > 8 || ctx->force_variant >= 0 || o.decode_form != JL_FORM_AUTO || o.pin_warps || o.pin_stages || o.pin_row_groups ||
+        (o.flags & JL_FLAG_DECODE_CONCURRENT))
+        return false;
+    // Small calls stay with a CTA per token: the tiles fetched again are few, and with x given their one launch (wide, fused)
+    // beats prep + multi. Measured, one call after the other: 9.4 against 12 us for 2..3 tokens of 4096 x 4096, 14.8 against 15.5
+    // for 5, 9.5 against 15 for 2 of 8192 x 2048, 17.0 against 17.2 for 2 of 4096 x 14336; 14.8 against 12.5 for 2 of 14336 x 4096,
+    // 20.0 against 15.6 for 8 of 4096 x 4096. With the operand prepared both are one launch: only the smallest stay.
+    if ((long long)nrows * ntok <= 8192 || (have_x && (long long)nrows * ntok * nsb < 400000)) return false;
+    return !have_x || ctx->tuned.find(jl_tune_shape_key(JL_TYPE_Q4_K, nrows, nsb * 256, ntok)) == ctx->tuned.end();
+}
+
 static void q4k_fill_choice(const q4k_variant &v, int nrows, int nsb, int ntok, jl_choice *c) {
     const int wpr = v.warps / v.rg;
     c->kernel = JL_K_MMA; c->form = v.form; c->warps = v.warps; c->stages = v.stages; c->rows_per_cta = 16 * v.rg;
@@ -733,6 +914,16 @@ int jl_gemv_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, jl_ch
             c.grid = (nrows + c.rows_per_cta - 1) / c.rows_per_cta * (ntok == 1 ? 1 : (ntok + 3) / 4);
         }
     } else {
+        if (q4k_use_multi(ctx, nrows, k / 256, ntok, true)) {
+            c.kernel = JL_K_MMA; c.form = JL_FORM_SPLIT; c.rows_per_cta = 16 * q4k_multi_rg(nrows);
+            c.warps = Q4KM_WPR * q4k_multi_rg(nrows) + 1; c.stages = 3;
+            c.split_k = Q4KM_WPR < k / 256 ? Q4KM_WPR : k / 256;
+            c.tile_m = 16; c.tile_n = 8; c.tile_k = 32;
+            c.grid = (nrows + c.rows_per_cta - 1) / c.rows_per_cta;
+            c.launches = 2;
+            *out = c;
+            return JL_OK;
+        }
         const int idx = q4k_pick(ctx, nrows, k / 256, ntok, true);
         if (idx < 0) return JL_DECLINED;
         q4k_fill_choice(q4k_variants[idx], nrows, k / 256, ntok, &c);
@@ -769,14 +960,14 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
                               "(jl_reserve sizes it)", ctx->scratch_cap, k, ntok, need);
         uint8_t *scratch = (uint8_t *)ctx->scratch;
         const bool prepared = x_dev == nullptr;   // the caller's kernels wrote the operand into the scratch already
-        const int idx = q4k_pick(ctx, nrows, nsb, ntok, !prepared);
-        if (idx < 0) return jl_set_err(ctx, JL_DECLINED, "no decode variant fits %d x %d", nrows, k);
-        const q4k_variant &v = q4k_variants[idx];
+        const bool multi = q4k_use_multi(ctx, nrows, nsb, ntok, !prepared);
+        const int idx = multi ? -1 : q4k_pick(ctx, nrows, nsb, ntok, !prepared);
+        if (!multi && idx < 0) return jl_set_err(ctx, JL_DECLINED, "no decode variant fits %d x %d", nrows, k);
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
         const int nattr = (ctx->opts.flags & JL_FLAG_NO_PDL) ? 0 : 1;
-        const bool converts = v.form == JL_FORM_FUSED || v.form == JL_FORM_WIDE;   // the kernel reads x itself
+        const bool converts = !multi && (q4k_variants[idx].form == JL_FORM_FUSED || q4k_variants[idx].form == JL_FORM_WIDE);   // the kernel reads x itself
         if (!converts && !prepared) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((nsb + 3) / 4, ntok); cfg.blockDim = dim3(128); cfg.stream = s;
@@ -784,6 +975,22 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
             JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, q4k_xprep_kernel, x_dev, scratch, nsb, ntok));
             ctx->st.launches++;
         }
+        if (multi) {
+            const int mrg = q4k_multi_rg(nrows);
+            const q4k_multi_form &mf = q4k_multi[mrg - 1][ntok];
+            if (!(ctx->multi_ready >> (mrg * 9 + ntok) & 1)) {       // once per context and form, not on every call
+                JL_CUDA(ctx, cudaFuncSetAttribute((const void *)mf.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, mf.smem));
+                ctx->multi_ready |= 1u << (mrg * 9 + ntok);
+            }
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((nrows + 16 * mrg - 1) / (16 * mrg)); cfg.blockDim = dim3((Q4KM_WPR * mrg + 1) * 32);
+            cfg.dynamicSmemBytes = mf.smem; cfg.stream = s; cfg.attrs = at; cfg.numAttrs = nattr;
+            JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, mf.fn, w->map_sb16, expert * nrows, (const uint8_t *)scratch, out_dev, nrows, nsb,
+                                            ctx->dev_status));
+            ctx->st.launches++;
+            return JL_OK;
+        }
+        const q4k_variant &v = q4k_variants[idx];
         const void *xsrc = converts ? (const void *)x_dev : (const void *)scratch;
         const size_t smem = q4k_variant_smem(v, nsb);
         if (smem > 48 * 1024)

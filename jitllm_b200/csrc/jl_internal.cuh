@@ -115,6 +115,7 @@ struct jl_ctx {
     void *x_dev; size_t x_cap;
     void *o_dev; size_t o_cap;
     void *scratch; size_t scratch_cap;
+    uint32_t multi_ready;               // forms of the 2..8-token decode kernel whose shared memory has been allowed
     // workspace of the Q6_K batch kernel, apart from the scratch (whose prepared operands outlive a call): sized for
     // what jl_reserve and the Q6_K uploads have asked for. q6k_done orders calls that come on another stream.
     void *q6k_work; size_t q6k_cap;

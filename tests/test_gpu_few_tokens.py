@@ -1,0 +1,86 @@
+"""A few tokens at a time: the Q4_K decode kernel that keeps 2..8 tokens inside a task, and the mixture layer's decode path."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import nmse, parity_err
+from jitllm_b200 import ACT_SILU, ACT_SWIGLU_OAI, MXFP4, Q4_K, Device, _lib, synth
+
+pytestmark = pytest.mark.gpu
+BAR = 2e-3
+
+
+# sizes that go to the kernel (rows x tokens x super-blocks of 400000 and more): one super-block, not a multiple of a row group's four
+# warps; ragged last row groups; the rows from which two row groups share a CTA (9472), one above and one group below
+@pytest.mark.parametrize("nrows,k,ntok", [(50001, 256, 8), (70001, 768, 2), (9472, 2816, 4), (9473, 4096, 3), (2048, 14336, 6), (1700, 14336, 5),
+                                          (9456, 1792, 7), (4099, 5120, 5)])
+def test_q4k_tokens_inside_the_task(orc, nrows, k, ntok):
+    rng = synth.rng_for(0xB800 + nrows + k + ntok)
+    w, x = synth.q4k_matrix(rng, nrows, k), synth.activations(rng, ntok, k)
+    st = torch.cuda.current_stream().cuda_stream
+    with Device(0) as d:
+        d.Reserve(nrows, k, ntok)
+        h = d.Upload(Q4_K, w, nrows, k)
+        xd, out = torch.from_numpy(x).cuda(), torch.full((ntok, nrows), float("nan"), device="cuda")
+        ch = d.Select(Q4_K, nrows, k, ntok)
+        assert ch.grid == -(-nrows // ch.rows_per_cta)             # the CTAs do not repeat per token
+        d.MatMulDev(out, h, xd, ntok, st)
+        one = torch.empty(ntok, nrows, device="cuda")
+        for i in range(ntok):
+            d.MatVecDev(one[i], h, xd[i], 1, st)
+        torch.cuda.synchronize()
+        assert d.StatusPoll()
+        got, ref = out.cpu().numpy(), orc.matmul_f64(Q4_K, w, x, nrows, k, ntok)
+        assert np.isfinite(got).all() and nmse(got, ref) < 1e-8
+        # the same integers per super-block as one token at a time; only the order of the f32 sums over super-blocks may differ
+        assert parity_err(got, one.cpu().numpy()) <= (k / 256 + 4) * 2.0 ** -23
+
+
+def _bank(dev, rng, E, H, F):
+    raw = [synth.mxfp4_matrix(rng, E * r, k) for r, k in ((F, H), (F, H), (H, F))]
+    return raw, [dev.Upload(MXFP4, w, r, k, E) for w, (r, k) in zip(raw, ((F, H), (F, H), (H, F)))]
+
+
+# one pair and the most (32); blocks left over in a unit of four; more experts a token than warps; rows too many to stage
+@pytest.mark.parametrize("E,K,H,F,ntok,act", [(1, 1, 64, 64, 1, 0), (8, 2, 192, 320, 7, 1), (32, 4, 2880, 2880, 1, 1), (32, 32, 64, 128, 1, 0),
+                                              (16, 16, 128, 2112, 2, 0), (4, 4, 704, 64, 8, 1)])
+@pytest.mark.parametrize("h_dtype", ["f32", "bf16", "f16"])
+def test_mixture_of_a_few_pairs(orc, E, K, H, F, ntok, act, h_dtype):
+    rng = synth.rng_for(0xB900 + E + K + H + F + ntok)
+    with Device(0) as dev:
+        dev.MoeReserve(ntok, E, K, H, F)
+        raw, banks = _bank(dev, rng, E, H, F)
+        bias = [rng.standard_normal((E, n)).astype(np.float32) for n in (F, F, H)]
+        bt = [torch.from_numpy(b).cuda() for b in bias]
+        d = _lib.MoeDesc(struct_size=C.sizeof(_lib.MoeDesc), type=MXFP4, n_expert=E, top_k=K, hidden=H, ffn=F,
+                         act=ACT_SWIGLU_OAI if act else ACT_SILU, norm=1, scale=1.0, gate=banks[0].handle, up=banks[1].handle,
+                         down=banks[2].handle, gate_bias=bt[0].data_ptr(), up_bias=bt[1].data_ptr(), down_bias=bt[2].data_ptr())
+        h = torch.from_numpy(synth.activations(rng, ntok, H) * np.float32(0.25)).cuda().to(getattr(torch, dict(f32="float32", bf16="bfloat16", f16="float16")[h_dtype]))
+        logits = torch.from_numpy(synth.activations(rng, ntok, E)).cuda()
+        base = torch.randn(ntok, H, device="cuda")
+        out, sel, wt = base.clone(), torch.empty(ntok, K, dtype=torch.int32, device="cuda"), torch.empty(ntok, K, device="cuda")
+        st = torch.cuda.current_stream().cuda_stream
+        dev.MoeDev(out, h, logits, ntok, d, sel, wt, st)
+        again = base.clone()
+        dev.MoeDev(again, h, logits, ntok, d, sel, wt, st)
+        torch.cuda.synchronize()
+        assert torch.equal(out, again)                                  # fixed order
+        hf = h.float().cpu().numpy()
+        ref = orc.moe_layer(hf, MXFP4, *raw, sel.cpu().numpy(), wt.cpu().numpy(), E, H, F, act_kind=d.act, bgate=bias[0], bup=bias[1], bdown=bias[2])
+        assert parity_err((out - base).cpu().numpy(), ref) <= 1e-4      # f16 hi + lo per 64 elements and f32 sums; the subtraction's rounding
+        # given ids: rows are written, an id outside the bank leaves its row alone
+        ids = torch.tensor([(3 * i + 1) % E for i in range(ntok)], dtype=torch.int32, device="cuda")
+        if ntok > 1:
+            ids[1] = -1
+        y = torch.full((ntok, H), 7.0, device="cuda")
+        dev.MoeExpertsDev(y, h, ids, ntok, d, st)
+        torch.cuda.synchronize()
+        for i in range(ntok):
+            if int(ids[i]) < 0:
+                assert bool((y[i] == 7.0).all())
+                continue
+            one = orc.moe_layer(hf[i:i + 1], MXFP4, *raw, ids[i:i + 1].cpu().numpy().reshape(1, 1), np.ones((1, 1), np.float32), E, H, F,
+                                act_kind=d.act, bgate=bias[0], bup=bias[1], bdown=bias[2])
+            assert parity_err(y[i:i + 1].cpu().numpy(), one) <= 1e-4
