@@ -127,6 +127,8 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const uint8_t *__restric
 // (q - 32) x is weighted by d * sc, which f32 holds exactly, so no weight is rounded at all. NT tokens share the codes.
 // Bound by what is in flight: a lane that read 2-byte words of the 210-byte blocks took 38.0 us for one token of 4096 x 14336;
 // the resident 208-byte blocks (see jl_weight) are read in 16-byte words, R x 58 bytes a thread at a time: 19.8 us, 2.4 TB/s.
+// R is 4 for every token count: the activations' loads (64 floats a unit and token) are then shared by four rows (with two, 4
+// tokens of 14336 x 4096 took 70 us, with four 44; a warp per row took 53).
 __device__ __forceinline__ void q6k_fma2(float2 &acc, float2 a, float2 b) {
     asm("{\n\t.reg .b64 ra, rb, rc;\n\t"
         "mov.b64 ra, {%2, %3};\n\t"
@@ -909,9 +911,9 @@ int jl_gemv_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, jl_ch
         c.kernel = JL_K_SIMT; c.warps = 8; c.rows_per_cta = 8; c.split_k = 1;
         c.grid = (nrows + 7) / 8 * ntok;
         c.launches = 1;
-        if (type == JL_TYPE_Q6_K) {                    // a block of threads per 4 rows (one token) or per 2 rows x 4 tokens
-            c.warps = min(8, (k / 64 + 31) / 32); c.rows_per_cta = ntok == 1 ? 4 : 2; c.split_k = 1;
-            c.grid = (nrows + c.rows_per_cta - 1) / c.rows_per_cta * (ntok == 1 ? 1 : (ntok + 3) / 4);
+        if (type == JL_TYPE_Q6_K) {                    // a block of threads per 4 rows x up to 4 tokens
+            c.warps = min(8, (k / 64 + 31) / 32); c.rows_per_cta = 4; c.split_k = 1;
+            c.grid = (nrows + 3) / 4 * ((ntok + 3) / 4);
         }
     } else {
         if (q4k_use_multi(ctx, nrows, k / 256, ntok, true)) {
@@ -1012,7 +1014,8 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
             const uint16_t *d = reinterpret_cast<const uint16_t *>(scales);
             const int threads = min(256, (k / 64 + 31) / 32 * 32);            // a thread per unit of the row, up to 256
             if (ntok == 1) gemv_q6k_kernel<4, 1><<<dim3((nrows + 3) / 4, 1), threads, 0, s>>>(data, d, x_dev, out_dev, nrows, k, ntok);
-            else gemv_q6k_kernel<2, 4><<<dim3((nrows + 1) / 2, (ntok + 3) / 4), threads, 0, s>>>(data, d, x_dev, out_dev, nrows, k, ntok);
+            else if (ntok == 2) gemv_q6k_kernel<4, 2><<<dim3((nrows + 3) / 4, 1), threads, 0, s>>>(data, d, x_dev, out_dev, nrows, k, ntok);
+            else gemv_q6k_kernel<4, 4><<<dim3((nrows + 3) / 4, (ntok + 3) / 4), threads, 0, s>>>(data, d, x_dev, out_dev, nrows, k, ntok);
         }
         else if (w->type == JL_TYPE_Q5_K) JL_ROWK(gemv_q5k_kernel);
         else if (w->type == JL_TYPE_Q4_0) JL_ROWK45(JL_TYPE_Q4_0);
