@@ -12,8 +12,7 @@
 // two and split x = hi + lo into two f16 rows, one MMA column each, so ~22 bits of every activation take
 // part; the 8 columns serve four tokens; 1 / scale of the span folds in with the block scales. Warps of a
 // CTA take different spans of the same 16 rows and meet in shared memory in fixed order (bit-stable).
-#include "jl_internal.cuh"
-#include <cuda_fp16.h>
+#include "mxfp4_dot.cuh"
 
 // scratch: f16 rows [2 * ntok][k] (hi, lo of each token), then f32 [ntok][k / 64] (1 / scale of each span)
 size_t jl_gemv_mxfp4_scratch_bytes(int k, int ntok) {
@@ -29,32 +28,13 @@ __global__ void __launch_bounds__(128) mx_xprep_kernel(const float *__restrict__
     const int lane = threadIdx.x & 31, sp = blockIdx.x * 4 + (threadIdx.x >> 5), tok = blockIdx.y, nspan = k / 64;
     if (sp >= nspan) return;
     const float2 v = __ldg(reinterpret_cast<const float2 *>(X + (size_t)tok * k + (size_t)sp * 64) + lane);
-    float amax = fmaxf(fabsf(v.x), fabsf(v.y));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    int sh = 14 - ((int)((__float_as_uint(amax) >> 23) & 0xFF) - 127);
-    if (amax == 0.f || !(amax < __int_as_float(0x7f800000))) sh = 0;
-    sh = max(-100, min(100, sh));
-    const float scale = __uint_as_float((uint32_t)(127 + sh) << 23);
-    const float a = v.x * scale, b = v.y * scale;
-    const __half2 hh = __floats2half2_rn(a, b);
-    const float2 back = __half22float2(hh);
-    const __half2 ll = __floats2half2_rn(a - back.x, b - back.y);
+    __half2 hh, ll;
+    const float inv = mx_split_span(v, hh, ll);
     __half2 *hi = reinterpret_cast<__half2 *>(xh + (size_t)(2 * tok) * k + (size_t)sp * 64);
     hi[lane] = hh;
     reinterpret_cast<__half2 *>(xh + (size_t)(2 * tok + 1) * k + (size_t)sp * 64)[lane] = ll;
-    if (lane == 0) inv_scale[(size_t)tok * nspan + sp] = __uint_as_float((uint32_t)(127 - sh) << 23);
+    if (lane == 0) inv_scale[(size_t)tok * nspan + sp] = inv;
 }
-
-__device__ __forceinline__ void mx_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                       uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// four codes in the HIGH nibbles of v's bytes -> the high bytes of their f16 images
-__device__ __forceinline__ uint32_t mx_hbytes(uint32_t v) { return ((v & 0x70707070u) >> 3) | (v & 0x80808080u); }
 
 // grid (row groups of 16, token groups of 4); WARPS warps split the row's 64-element spans.
 template <int WARPS>
@@ -124,18 +104,10 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_mxfp4_mma_kernel(const uint8_
             float sa = 0.f, sb = 0.f;
 #pragma unroll
             for (int b = 0; b < 2; b++) {
-                const uint32_t hla = mx_hbytes(ua[u][b] << 4), hha = mx_hbytes(ua[u][b]);     // low / high nibbles of row g
-                const uint32_t hlb = mx_hbytes(ub[u][b] << 4), hhb = mx_hbytes(ub[u][b]);     // ... of row g + 8
                 float c[4] = {0.f, 0.f, 0.f, 0.f};
-                // k-slots (2t, 2t+1 | 2t+8, 2t+9) = elements (4t, 4t+1 | 4t+2, 4t+3), then the same + 16
-                mx_mma(c, __byte_perm(hla, 0u, 0x1404), __byte_perm(hlb, 0u, 0x1404), __byte_perm(hla, 0u, 0x3424),
-                       __byte_perm(hlb, 0u, 0x3424), x0[u][b].x, x0[u][b].y);
-                mx_mma(c, __byte_perm(hha, 0u, 0x1404), __byte_perm(hhb, 0u, 0x1404), __byte_perm(hha, 0u, 0x3424),
-                       __byte_perm(hhb, 0u, 0x3424), x1[u][b].x, x1[u][b].y);
-                // 2^(e - 127) * 2^14 as an f32 (an all-zero block may carry any byte: keep the exponent field legal)
-                const uint32_t e_a = min((ce_a[u] >> (8 * b)) & 0xFFu, 240u), e_b = min((ce_b[u] >> (8 * b)) & 0xFFu, 240u);
-                sa = fmaf(c[0] + c[1], __uint_as_float((e_a + 14u) << 23), sa);     // hi + lo columns of token t
-                sb = fmaf(c[2] + c[3], __uint_as_float((e_b + 14u) << 23), sb);
+                mx_block(c, ua[u][b], ub[u][b], x0[u][b], x1[u][b]);
+                sa = fmaf(c[0] + c[1], mx_block_scale(ce_a[u] >> (8 * b)), sa);     // hi + lo columns of token t
+                sb = fmaf(c[2] + c[3], mx_block_scale(ce_b[u] >> (8 * b)), sb);
             }
             acc_a = fmaf(sa, is[u], acc_a);
             acc_b = fmaf(sb, is[u], acc_b);

@@ -270,6 +270,7 @@ __device__ __forceinline__ float moe_act(int kind, float g, float u) {
 }
 
 #include "moe_bs.cuh"
+#include "moe_dec.cuh"
 
 template <int NT, int SA, int SB>
 struct moe_smem {
@@ -726,6 +727,27 @@ static int moe_dev_locked(jl_ctx *ctx, float *out_dev, const void *h_dev, int h_
     at[0].val.programmaticStreamSerializationAllowed = 1;
     const int nattr = (ctx->opts.flags & JL_FLAG_NO_PDL) ? 0 : 1;
     auto cfg_of = [&](dim3 g, dim3 b) { cudaLaunchConfig_t c = {}; c.gridDim = g; c.blockDim = b; c.stream = s; c.attrs = at; c.numAttrs = nattr; return c; };
+    if (np <= (d->arm == JL_MOE_ARM_EXACT ? min(32, 2 * E) : 8) && d->arm != JL_MOE_ARM_BLOCK_SCALED) {
+        // few pairs: matrix-vector products of the chosen experts (moe_dec.cuh says where the lines lie), the same or finer
+        // arithmetic than either arm
+        moe_dec_params q = {};
+        q.n_expert = E; q.top_k = K; q.hidden = H; q.ffn = F; q.act = d->act;
+        q.cg = wg->data; q.cu = wu->data; q.cd = wd->data; q.eg = wg->scales; q.eu = wu->scales; q.ed = wd->scales;
+        q.eg_stride = wg->scale_stride; q.ed_stride = wd->scale_stride;
+        q.bg = d->gate_bias; q.bu = d->up_bias; q.bd = d->down_bias;
+        q.sel = sel; q.wt = given_ids ? nullptr : wt; q.out = out_dev;
+        q.xh = xs; q.xinv = y; q.ah = as; q.ainv = act;
+        const int route_blocks = given_ids ? 0 : (ntok + 3) / 4;
+        cudaLaunchConfig_t c = cfg_of(dim3(route_blocks + (H / 64 * ntok + 3) / 4), dim3(128));
+        JL_CUDA(ctx, cudaLaunchKernelEx(&c, moe_dec_prep_kernel, logits_dev, d->router_bias, d->sel_bias, ntok, E, K, d->norm, d->scale, sel, wt,
+                                        route_blocks, h_dev, h_dtype, xs, y, H));
+        c = cfg_of(dim3(F / 64, np), dim3(MXD_WARPS * 32));
+        JL_CUDA(ctx, cudaLaunchKernelEx(&c, moe_dec_gate_up_kernel, q));
+        c = cfg_of(dim3(H / 16, ntok), dim3(MXD_WARPS * 32));
+        JL_CUDA(ctx, cudaLaunchKernelEx(&c, moe_dec_down_kernel, q));
+        ctx->st.launches += 3;
+        return JL_OK;
+    }
     {
         // (Router and sort as ONE launch were built twice and measured slower: a single CTA routing all tokens, +65 us
         // per layer -- the f64 softmax of 256 tokens on one SM; and the router's last CTA, by ticket, sorting, +7 us.

@@ -45,7 +45,7 @@ def _bank(dev, rng, E, H, F):
 
 # one pair and the most (32); blocks left over in a unit of four; more experts a token than warps; rows too many to stage
 @pytest.mark.parametrize("E,K,H,F,ntok,act", [(1, 1, 64, 64, 1, 0), (8, 2, 192, 320, 7, 1), (32, 4, 2880, 2880, 1, 1), (32, 32, 64, 128, 1, 0),
-                                              (16, 16, 128, 2112, 2, 0), (4, 4, 704, 64, 8, 1)])
+                                              (16, 16, 128, 2112, 2, 0), (16, 4, 704, 64, 8, 1)])
 @pytest.mark.parametrize("h_dtype", ["f32", "bf16", "f16"])
 def test_mixture_of_a_few_pairs(orc, E, K, H, F, ntok, act, h_dtype):
     rng = synth.rng_for(0xB900 + E + K + H + F + ntok)
