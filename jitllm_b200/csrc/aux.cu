@@ -242,57 +242,65 @@ __device__ __forceinline__ void aux_bf16x8(const uint4 &v, float *f) {
     }
 }
 
-// D (16 x 8, f32) += A (16 x 16 bf16, row) * B (16 x 8 bf16, col).
-__device__ __forceinline__ void aux_mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                             uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// D (16 x 8, f32) += A (16 x 16 bf16, row) * B (16 x 8 bf16, col), with rows 8..15 of A zero: their accumulators stay zero and
+// are not kept.
+__device__ __forceinline__ void aux_mma_bf16(float (&d)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+    float unused0, unused1;
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(unused0), "=f"(unused1)
+                 : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(d[0]), "f"(d[1]), "f"(0.f), "f"(0.f));
 }
 
-#ifndef ATT_MIN_CTAS
-#define ATT_MIN_CTAS 5          // 96 registers: five CTAs per SM (shared memory would allow six, but at 80 registers the kernel spills)
-#endif
+// One CTA takes `per` chunks of 64 positions, a warp of it 16 positions of every chunk, with its own running (max, sum, weighted V)
+// and its own two-stage cp.async ring: no warp waits for another before the end of the CTA's positions. With one chunk to a
+// CTA (the small batches' form still) a batch of 64 at 2049 positions was 16,900 CTAs, each a load, five barriers, a
+// record, a fence and a ticket, and the cache came in at 3.9 TB/s; several chunks to a CTA keep the next tile on its way
+// while one is used and write a fraction of the records.
+#define ATT_STAGES 2
+#define ATT_WARP_TILE (2 * 16 * ATT_ROW)              // 16 rows of K, 16 of V
+#define ATT_SMEM (4 * ATT_STAGES * ATT_WARP_TILE)
 template <int G>
-__global__ void __launch_bounds__(128, ATT_MIN_CTAS) aux_attn_decode_kernel(float *out, uint8_t *operand, const __nv_bfloat16 *q,
+__global__ void __launch_bounds__(128, 3) aux_attn_decode_kernel(float *out, uint8_t *operand, const __nv_bfloat16 *q,
                                                               const __nv_bfloat16 *k_cache, const __nv_bfloat16 *v_cache,
                                                               const long long *pos_dev, float *part, unsigned *tickets, int hkv,
-                                                              int max_len, int nsplit) {
+                                                              int max_len, int nsplit, int per) {
     constexpr int HDR = (2 * G + 3) & ~3;              // max[G], sum[G], padded so that the V part is 16-byte aligned
     constexpr int STRIDE = HDR + G * ATT_D;
-    // K and V tiles of the chunk, staged with coalesced 16-byte loads (all in flight at once); the
-    // cross-group reduction buffer red[8][G][128] reuses the tiles once they have been consumed.
-    __shared__ __align__(16) uint8_t tiles[2 * ATT_CHUNK * ATT_ROW];
-    static_assert(4 * G * ATT_D * 4 <= 2 * ATT_CHUNK * ATT_ROW, "reduction buffer must fit in the tiles");
+    extern __shared__ __align__(16) uint8_t tiles[];   // the warps' rings; the cross-warp sum red[4][G][128] reuses them
+    static_assert(4 * G * ATT_D * 4 <= ATT_SMEM, "reduction buffer must fit in the tiles");
     __shared__ float mred[4][G], lred[4][G];
     __shared__ unsigned last;
     const int split = blockIdx.x, kv = blockIdx.y, row = blockIdx.z, t = threadIdx.x, hq = hkv * G;
     AUX_PDL();
     long long len = *pos_dev + 1;
     if (len > max_len) len = max_len;
-    const int s0 = split * ATT_CHUNK;
-    const int cnt = len - s0 < 0 ? 0 : (len - s0 > ATT_CHUNK ? ATT_CHUNK : (int)(len - s0));
+    const int span = ATT_CHUNK * per, s0 = split * span;
+    const int cnt = len - s0 < 0 ? 0 : (len - s0 > span ? span : (int)(len - s0));
     float *my = part + (((size_t)row * hkv + kv) * nsplit + split) * STRIDE;
     if (cnt > 0) {
         const size_t base_row = ((size_t)row * hkv + kv) * max_len + s0;
-        const uint4 *kg = (const uint4 *)(k_cache + base_row * ATT_D), *vg = (const uint4 *)(v_cache + base_row * ATT_D);
-        uint4 kreg[8], vreg[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {                            // 1024 16-byte pieces per tile, 8 per thread
-            const int piece = i * 128 + t;
-            kreg[i] = (piece >> 4) < cnt ? kg[piece] : make_uint4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int piece = i * 128 + t;
-            vreg[i] = (piece >> 4) < cnt ? vg[piece] : make_uint4(0, 0, 0, 0);
-        }
-        // Scores and the weighted sum of V run on the tensor cores (mma.sync m16n8k16, bf16 in, f32 accumulate): the M
-        // rows are the group's G query heads (rows G..15 are zero), a warp takes 16 of the chunk's 64 positions. q and
-        // the cached K, V are bf16 as stored, so the products are exact; the softmax weights go in as a bf16 pair
-        // (value + what the first rounding left: 16 significant bits). Per byte of cache this is a quarter of the
-        // instructions of a scalar loop, which is what bounded the kernel at batch 64.
         const int warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
+        const int ntile = cnt > warp * 16 ? (cnt - warp * 16 + ATT_CHUNK - 1) / ATT_CHUNK : 0;
+        const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tiles) + warp * ATT_STAGES * ATT_WARP_TILE;
+        // tile i of the warp: positions 64 i + 16 warp .. + 15, K rows then V rows; rows past cnt arrive as zeros
+        auto issue = [&](int i) {
+            const uint32_t dst = ring + (i % ATT_STAGES) * ATT_WARP_TILE;
+            const int p = i * ATT_CHUNK + warp * 16;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int piece = j * 32 + lane, r = piece >> 4, c = piece & 15;
+                const size_t at = (base_row + min(p + r, cnt - 1)) * ATT_D + c * 8;
+                const int bytes = p + r < cnt ? 16 : 0;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * ATT_ROW + c * 16), "l"(k_cache + at), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (16 + r) * ATT_ROW + c * 16), "l"(v_cache + at), "r"(bytes) : "memory");
+            }
+        };
+        if (ntile > 0) issue(0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        // Scores and the weighted sum of V run on the tensor cores (mma.sync m16n8k16, bf16 in, f32 accumulate): the M
+        // rows are the group's G query heads (rows G..15 are zero). q and the cached K, V are bf16 as stored, so the
+        // products are exact; the softmax weights go in as a bf16 pair (value + what the first rounding left: 16
+        // significant bits).
         uint32_t qa[8][2];                                      // A fragments of q: k-step s covers dims 16 s .. 16 s + 15
         {
             const uint32_t *qrow = reinterpret_cast<const uint32_t *>(q + ((size_t)row * hq + kv * G + (g < G ? g : 0)) * ATT_D);
@@ -302,97 +310,98 @@ __global__ void __launch_bounds__(128, ATT_MIN_CTAS) aux_attn_decode_kernel(floa
                 qa[ks][1] = g < G ? __ldg(qrow + ks * 8 + 4 + tq) : 0u;        // dims 16 ks + 8 + 2 tq, + 1
             }
         }
+        float M = -INFINITY, l = 0.f;                           // of head g over the warp's positions so far (l: this lane's share)
+        float oacc[16][2];                                      // O[g][8 j + 2 tq, + 1]
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int piece = i * 128 + t;
-            *(uint4 *)(tiles + (piece >> 4) * ATT_ROW + (piece & 15) * 16) = kreg[i];
-            *(uint4 *)(tiles + (ATT_CHUNK + (piece >> 4)) * ATT_ROW + (piece & 15) * 16) = vreg[i];
-        }
-        __syncthreads();
-        const uint32_t tiles_s = (uint32_t)__cvta_generic_to_shared(tiles);
-        const int p0 = warp * 16;                               // the warp's positions p0 .. p0 + 15 of the chunk
-        // S[h][pos]: two n-tiles of 8 positions; lane (g, tq) ends up with S[g][p0 + 8 nt + 2 tq, + 1]
-        float sacc[2][4];
+        for (int j = 0; j < 16; ++j) oacc[j][0] = oacc[j][1] = 0.f;
+#pragma unroll 1
+        for (int i = 0; i < ntile; ++i) {
+            __syncwarp();                                       // every lane is done with the stage that is refilled now
+            if (i + 1 < ntile) issue(i + 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            const uint32_t tile = ring + (i % ATT_STAGES) * ATT_WARP_TILE;
+            const int p = i * ATT_CHUNK + warp * 16;
+            // S[h][pos]: two n-tiles of 8 positions; lane (g, tq) ends up with S[g][p + 8 nt + 2 tq, + 1]
+            float sv[4];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
+            for (int nt = 0; nt < 2; ++nt) {
+                float sacc[2] = {0.f, 0.f};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) sacc[nt][e] = 0.f;
+                for (int kp = 0; kp < 4; ++kp) {                // two k-steps (32 dims) per ldmatrix.x4
+                    // matrices: K[8 nt + 0..7][dims 32 kp + 0..7 | 8..15 | 16..23 | 24..31]
+                    const uint32_t addr = tile + (8 * nt + (lane & 7)) * ATT_ROW + (32 * kp + 8 * (lane >> 3)) * 2;
+                    uint32_t b0, b1, b2, b3;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
+                    aux_mma_bf16(sacc, qa[2 * kp][0], qa[2 * kp][1], b0, b1);
+                    aux_mma_bf16(sacc, qa[2 * kp + 1][0], qa[2 * kp + 1][1], b2, b3);
+                }
 #pragma unroll
-            for (int kp = 0; kp < 4; ++kp) {                    // two k-steps (32 dims) per ldmatrix.x4
-                // matrices: K[p0 + 8 nt + 0..7][dims 32 kp + 0..7 | 8..15 | 16..23 | 24..31]
-                const uint32_t addr = tiles_s + (p0 + 8 * nt + (lane & 7)) * ATT_ROW + (32 * kp + 8 * (lane >> 3)) * 2;
-                uint32_t b0, b1, b2, b3;
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
-                aux_mma_bf16(sacc[nt], qa[2 * kp][0], 0u, qa[2 * kp][1], 0u, b0, b1);
-                aux_mma_bf16(sacc[nt], qa[2 * kp + 1][0], 0u, qa[2 * kp + 1][1], 0u, b2, b3);
+                for (int e = 0; e < 2; ++e) sv[2 * nt + e] = p + 8 * nt + 2 * tq + e < cnt ? sacc[e] * 0.08838834764831845f : -INFINITY;
             }
-        }
-        float sv[4];                                            // this lane's four scores of head g
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int pos = p0 + 8 * nt + 2 * tq + e;
-                sv[2 * nt + e] = pos < cnt ? sacc[nt][e] * 0.08838834764831845f : -INFINITY;
-            }
-        {
             float m = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            if (tq == 0 && g < G) mred[warp][g] = m;
-        }
-        __syncthreads();
-        const int gh = g < G ? g : 0;
-        const float M = fmaxf(fmaxf(mred[0][gh], mred[1][gh]), fmaxf(mred[2][gh], mred[3][gh]));
-        float pv[4], l = 0.f;
+            m = fmaxf(m, M);
+            const float keep = M > -INFINITY ? __expf(M - m) : 0.f;
+            M = m;
+            float pv[4];
+            l *= keep;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            pv[e] = (g < G && sv[e] > -INFINITY) ? __expf(sv[e] - M) : 0.f;
-            l += pv[e];
+            for (int e = 0; e < 4; ++e) {
+                pv[e] = (g < G && sv[e] > -INFINITY) ? __expf(sv[e] - M) : 0.f;
+                l += pv[e];
+            }
+            // A fragments of the weights: positions 2 tq, + 1 (a0) and 8 + 2 tq, + 1 (a2), as value + remainder
+            uint32_t ph[2], pl[2];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                const __nv_bfloat162 hi = __floats2bfloat162_rn(pv[2 * nt], pv[2 * nt + 1]);
+                const float2 hf = __bfloat1622float2(hi);
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(pv[2 * nt] - hf.x, pv[2 * nt + 1] - hf.y);
+                ph[nt] = *reinterpret_cast<const uint32_t *>(&hi);
+                pl[nt] = *reinterpret_cast<const uint32_t *>(&lo);
+            }
+            // O[h][dim] += P[h][pos] V[pos][dim]: sixteen n-tiles of 8 dims, two per ldmatrix.x4.trans
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { oacc[j][0] *= keep; oacc[j][1] *= keep; }
+#pragma unroll
+            for (int jp = 0; jp < 8; ++jp) {
+                // matrices: V[0..7][dims 16 jp + 0..7], V[8..15][same], V[0..7][dims 16 jp + 8..15], V[8..15][same]
+                const int mi = lane >> 3;
+                const uint32_t addr = tile + (16 + 8 * (mi & 1) + (lane & 7)) * ATT_ROW + (16 * jp + 8 * (mi >> 1)) * 2;
+                uint32_t b0, b1, b2, b3;
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
+                aux_mma_bf16(oacc[2 * jp], ph[0], ph[1], b0, b1);
+                aux_mma_bf16(oacc[2 * jp], pl[0], pl[1], b0, b1);
+                aux_mma_bf16(oacc[2 * jp + 1], ph[0], ph[1], b2, b3);
+                aux_mma_bf16(oacc[2 * jp + 1], pl[0], pl[1], b2, b3);
+            }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         l += __shfl_xor_sync(0xffffffffu, l, 1);
         l += __shfl_xor_sync(0xffffffffu, l, 2);
-        if (tq == 0 && g < G) lred[warp][g] = l;
-        // A fragments of the weights: positions p0 + 2 tq, + 1 (a0) and p0 + 8 + 2 tq, + 1 (a2), as value + remainder
-        uint32_t ph[2], pl[2];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            const __nv_bfloat162 hi = __floats2bfloat162_rn(pv[2 * nt], pv[2 * nt + 1]);
-            const float2 hf = __bfloat1622float2(hi);
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(pv[2 * nt] - hf.x, pv[2 * nt + 1] - hf.y);
-            ph[nt] = *reinterpret_cast<const uint32_t *>(&hi);
-            pl[nt] = *reinterpret_cast<const uint32_t *>(&lo);
-        }
-        // O[h][dim] += P[h][pos] V[pos][dim]: sixteen n-tiles of 8 dims, two per ldmatrix.x4.trans
-        float oacc[16][4];
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) oacc[j][e] = 0.f;
-#pragma unroll
-        for (int jp = 0; jp < 8; ++jp) {
-            // matrices: V[p0 + 0..7][dims 16 jp + 0..7], V[p0 + 8..15][same], V[p0 + 0..7][dims 16 jp + 8..15], V[p0 + 8..15][same]
-            const int mi = lane >> 3;
-            const uint32_t addr = tiles_s + (ATT_CHUNK + p0 + 8 * (mi & 1) + (lane & 7)) * ATT_ROW + (16 * jp + 8 * (mi >> 1)) * 2;
-            uint32_t b0, b1, b2, b3;
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
-            aux_mma_bf16(oacc[2 * jp], ph[0], 0u, ph[1], 0u, b0, b1);
-            aux_mma_bf16(oacc[2 * jp], pl[0], 0u, pl[1], 0u, b0, b1);
-            aux_mma_bf16(oacc[2 * jp + 1], ph[0], 0u, ph[1], 0u, b2, b3);
-            aux_mma_bf16(oacc[2 * jp + 1], pl[0], 0u, pl[1], 0u, b2, b3);
-        }
-        __syncthreads();                                        // tiles consumed (and lred complete): reuse them
-        if (t < G) {
-            my[t] = fmaxf(fmaxf(mred[0][t], mred[1][t]), fmaxf(mred[2][t], mred[3][t]));
-            my[G + t] = (lred[0][t] + lred[1][t]) + (lred[2][t] + lred[3][t]);
-        }
+        if (tq == 0 && g < G) { mred[warp][g] = M; lred[warp][g] = l; }
+        __syncthreads();                                        // every warp's tiles are consumed: reuse them
+        const int gh = g < G ? g : 0;
+        const float Mall = fmaxf(fmaxf(mred[0][gh], mred[1][gh]), fmaxf(mred[2][gh], mred[3][gh]));
+        const float scale = mred[warp][gh] > -INFINITY ? __expf(mred[warp][gh] - Mall) : 0.f;
         float(*red)[G][ATT_D] = (float(*)[G][ATT_D])tiles;      // red[warp][head][dim]
         if (g < G) {
 #pragma unroll
             for (int j = 0; j < 16; ++j)
-                *reinterpret_cast<float2 *>(&red[warp][g][8 * j + 2 * tq]) = make_float2(oacc[j][0], oacc[j][1]);
+                *reinterpret_cast<float2 *>(&red[warp][g][8 * j + 2 * tq]) = make_float2(oacc[j][0] * scale, oacc[j][1] * scale);
+        }
+        if (t < G) {
+            const float mt = fmaxf(fmaxf(mred[0][t], mred[1][t]), fmaxf(mred[2][t], mred[3][t]));
+            float lt = 0.f;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) lt += mred[w][t] > -INFINITY ? lred[w][t] * __expf(mred[w][t] - mt) : 0.f;
+            my[t] = mt;
+            my[G + t] = lt;
         }
         __syncthreads();
 #pragma unroll
@@ -409,7 +418,7 @@ __global__ void __launch_bounds__(128, ATT_MIN_CTAS) aux_attn_decode_kernel(floa
     if (!last) return;
     __threadfence();
     const float *base = part + ((size_t)row * hkv + kv) * nsplit * STRIDE;
-    const int nlive = (int)((len + ATT_CHUNK - 1) / ATT_CHUNK);   // chunks past the sequence hold nothing
+    const int nlive = (int)((len + span - 1) / span);             // splits past the sequence hold nothing
     // Merge: warp w takes heads w, w+4, ...; its lanes first scan the chunks' (max, sum) pairs side by side,
     // then each lane owns four output dims and walks the chunks in ascending order (bit-stable) with the
     // loads of eight chunks in flight at a time.
@@ -573,6 +582,18 @@ JL_EXPORT size_t jl_aux_attn_scratch_bytes(int n, int hq, int hkv, int max_len) 
     return aux_attn_ticket_bytes(n, hkv) + (size_t)n * hkv * nsplit * (((2 * g + 3) & ~3) + g * ATT_D) * sizeof(float);
 }
 
+template <typename... Args>
+static int aux_attn_launch(void (*kern)(Args...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess) { cudaGetLastError(); return JL_ECUDA; }
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = ATT_SMEM; cfg.stream = s; cfg.attrs = at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, args...) != cudaSuccess) { cudaGetLastError(); return JL_ECUDA; }
+    return JL_OK;
+}
+
 JL_EXPORT int jl_aux_attn_decode(float *out, void *operand_out, const void *q_bf16, const void *k_cache_bf16,
                                  const void *v_cache_bf16, const long long *pos_dev, void *scratch_zeroed_once, int n, int hq,
                                  int hkv, int d, int max_len, void *stream) {
@@ -581,7 +602,12 @@ JL_EXPORT int jl_aux_attn_decode(float *out, void *operand_out, const void *q_bf
     if (aux_misaligned(out) || aux_misaligned(operand_out) || aux_misaligned(q_bf16) || aux_misaligned(k_cache_bf16) ||
         aux_misaligned(v_cache_bf16) || aux_misaligned(scratch_zeroed_once))
         return JL_EINVAL;
-    const int g = hq / hkv, nsplit = (max_len + ATT_CHUNK - 1) / ATT_CHUNK;
+    // Chunks per CTA: as many as leave four waves of three CTAs to an SM, eight at most (a record and a ticket every 512
+    // positions are nothing any more); one where the sequences alone do not fill the GPU, since there the CTAs' own time is
+    // the call's.
+    const int g = hq / hkv, chunks = (max_len + ATT_CHUNK - 1) / ATT_CHUNK;
+    const long long fill = (long long)n * hkv * chunks / (148 * 3 * 4);
+    const int per = fill < 1 ? 1 : (fill > 8 ? 8 : (int)fill), nsplit = (chunks + per - 1) / per;
     if (operand_out && (g & 1)) return JL_EINVAL;      // a super-block of the operand is two heads
     unsigned *tickets = (unsigned *)scratch_zeroed_once;
     float *part = (float *)((uint8_t *)scratch_zeroed_once + aux_attn_ticket_bytes(n, hkv));
@@ -591,10 +617,10 @@ JL_EXPORT int jl_aux_attn_decode(float *out, void *operand_out, const void *q_bf
     const __nv_bfloat16 *q = (const __nv_bfloat16 *)q_bf16, *kc = (const __nv_bfloat16 *)k_cache_bf16,
                         *vc = (const __nv_bfloat16 *)v_cache_bf16;
     switch (g) {
-    case 1: return aux_launch(aux_attn_decode_kernel<1>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit);
-    case 2: return aux_launch(aux_attn_decode_kernel<2>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit);
-    case 4: return aux_launch(aux_attn_decode_kernel<4>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit);
-    case 8: return aux_launch(aux_attn_decode_kernel<8>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit);
+    case 1: return aux_attn_launch(aux_attn_decode_kernel<1>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
+    case 2: return aux_attn_launch(aux_attn_decode_kernel<2>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
+    case 4: return aux_attn_launch(aux_attn_decode_kernel<4>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
+    case 8: return aux_attn_launch(aux_attn_decode_kernel<8>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
     }
     return JL_ENOTSUP;
 }
