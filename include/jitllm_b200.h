@@ -365,6 +365,11 @@ int jl_aux_add_rmsnorm_gemm(float *x_io, const float *delta /* or NULL */, const
                             void *rows_f16, float *inv_scale, int n, int h, void *stream);
 int jl_aux_silu_mul(float *out /* or NULL when operand_out is given */, void *operand_out,
                     const float *gate_up /* [n][2*ffn] */, int n, int ffn, void *stream);
+/* SiLU*up of [n][2*ffn] as the GEMM's activation operand (jl_gemm_operand of a weight of width ffn; ffn % 256 == 0). */
+int jl_aux_silu_mul_gemm(void *rows_f16, float *inv_scale, const float *gate_up, int n, int ffn, void *stream);
+/* A prompt: row r of qkv is position r; k and v go to position r of each of the cache's first `slots` sequences. */
+int jl_aux_rope_prefill(void *q_out_bf16 /* [n][hq][d] */, const float *qkv, void *k_cache_bf16, void *v_cache_bf16, const float *cos_t,
+                        const float *sin_t, int n, int slots, int hq, int hkv, int d, int max_len, void *stream);
 int jl_aux_argmax(long long *out /* [n] */, const float *x /* [n][v] */, int n, int v, void *stream);
 int jl_aux_rope_kv(void *q_out_bf16, const float *qkv, void *k_cache_bf16, void *v_cache_bf16,
                    const long long *pos_dev, const float *cos_t, const float *sin_t, int n, int hq, int hkv, int d,

@@ -141,6 +141,8 @@ SYMBOLS = {
     "jl_matvec_q4k_noalloc": (_I, [_VP, _VP, _VP, _I, _I, _VP]),
     "jl_aux_add_rmsnorm": (_I, [_VP, _VP, _VP, C.c_float, _VP, _VP, _I, _I, _VP]),
     "jl_aux_silu_mul": (_I, [_VP, _VP, _VP, _I, _I, _VP]),
+    "jl_aux_silu_mul_gemm": (_I, [_VP, _VP, _VP, _I, _I, _VP]),
+    "jl_aux_rope_prefill": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP]),
     "jl_aux_argmax": (_I, [_VP, _VP, _I, _I, _VP]),
     "jl_aux_rope_kv": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _VP]),
     "jl_aux_attn_scratch_bytes": (C.c_size_t, [_I, _I, _I, _I]),

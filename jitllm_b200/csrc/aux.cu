@@ -198,6 +198,83 @@ __global__ void __launch_bounds__(256) aux_silu_mul_kernel(float *out, const flo
     }
 }
 
+// SiLU(gate) * up straight into the tcgen05 GEMM's activation operand (bit for bit what act_to_f16_kernel makes of the f32
+// rows): one CTA per row, the row in shared memory between the pass that finds its largest magnitude and the one that
+// writes the f16 hi / lo halves. Through f32 rows in memory the 1531 x 14336 rows of a prompt were written once and read
+// twice again (88 MB each) before the GEMM saw them.
+__global__ void __launch_bounds__(512) aux_silu_mul_gemm_kernel(__half *rows, float *inv_scale, const float *gu, int ffn) {
+    extern __shared__ float4 srow[];
+    __shared__ float red[16];
+    AUX_PDL();
+    const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float4 *g4 = (const float4 *)(gu + (size_t)row * 2 * ffn), *u4 = g4 + ffn / 4;
+    float amax = 0.f;
+    for (int i = threadIdx.x; i < ffn / 4; i += 512) {
+        const float4 g = g4[i], u = u4[i];
+        const float4 v = make_float4(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y,
+                                     g.z / (1.f + __expf(-g.z)) * u.z, g.w / (1.f + __expf(-g.w)) * u.w);
+        srow[i] = v;
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) red[warp] = amax;
+    __syncthreads();
+    amax = red[0];
+#pragma unroll
+    for (int i = 1; i < 16; ++i) amax = fmaxf(amax, red[i]);
+    const int e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 127;
+    int s = 14 - e;
+    if (amax == 0.f || !(amax < __int_as_float(0x7f800000))) s = 0;
+    s = max(-100, min(100, s));
+    const float scale = __uint_as_float((uint32_t)(127 + s) << 23);
+    if (threadIdx.x == 0) inv_scale[row] = __uint_as_float((uint32_t)(127 - s) << 23);
+    __half *hi = rows + (size_t)(2 * row) * ffn, *lo = hi + ffn;
+    for (int i = threadIdx.x; i < ffn / 4; i += 512) {
+        const float4 v = srow[i];                                // this thread's own writes
+        const float a[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+        uint32_t hw[2], lw[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const __half2 hh = __floats2half2_rn(a[2 * j], a[2 * j + 1]);
+            const float2 back = __half22float2(hh);
+            const __half2 ll = __floats2half2_rn(a[2 * j] - back.x, a[2 * j + 1] - back.y);
+            hw[j] = *reinterpret_cast<const uint32_t *>(&hh);
+            lw[j] = *reinterpret_cast<const uint32_t *>(&ll);
+        }
+        *reinterpret_cast<uint2 *>(hi + (size_t)i * 4) = make_uint2(hw[0], hw[1]);
+        *reinterpret_cast<uint2 *>(lo + (size_t)i * 4) = make_uint2(lw[0], lw[1]);
+    }
+}
+
+// A prompt's RoPE and cache fill: row r of qkv [n][(hq + 2 hkv) * d] f32 is position r. q_out [n][hq][d] bf16 (rotated); k
+// (rotated) and v go to position r of every one of the `slots` sequences of the caches [slots][hkv][max_len][d]. One CTA per
+// position walks the whole row with coalesced 8-byte loads: one pass over what eight elementwise kernels moved.
+__global__ void __launch_bounds__(256) aux_rope_prefill_kernel(__nv_bfloat16 *q_out, const float *qkv, __nv_bfloat16 *k_cache,
+                                                                __nv_bfloat16 *v_cache, const float *cos_t, const float *sin_t, int slots,
+                                                                int hq, int hkv, int d, int max_len) {
+    AUX_PDL();
+    const int pos = blockIdx.x, half = d / 2, heads = hq + 2 * hkv;
+    const float2 *src = (const float2 *)(qkv + (size_t)pos * heads * d);
+    for (int i = threadIdx.x; i < heads * half; i += 256) {
+        const int hd = i / half, j = i - hd * half;
+        const float2 v = src[i];
+        __nv_bfloat162 o;
+        if (hd < hq + hkv) {
+            const float c = cos_t[(size_t)pos * half + j], s = sin_t[(size_t)pos * half + j];
+            o = __floats2bfloat162_rn(v.x * c - v.y * s, v.x * s + v.y * c);
+        } else {
+            o = __floats2bfloat162_rn(v.x, v.y);
+        }
+        if (hd < hq) {
+            ((__nv_bfloat162 *)(q_out + ((size_t)pos * hq + hd) * d))[j] = o;
+        } else {
+            __nv_bfloat16 *cache = hd < hq + hkv ? k_cache : v_cache;
+            const int kv = hd < hq + hkv ? hd - hq : hd - hq - hkv;
+            for (int b = 0; b < slots; ++b) ((__nv_bfloat162 *)(cache + (((size_t)b * hkv + kv) * max_len + pos) * d))[j] = o;
+        }
+    }
+}
+
 // qkv [n][(hq + 2 hkv) * d] f32 -> q_out [n][hq][d] bf16 (rotated), k (rotated) and v appended to the
 // caches [n][hkv][max_len][d] bf16 at position *pos. Adjacent-pair rotation; cos/sin are [max_len][d/2].
 __global__ void __launch_bounds__(64) aux_rope_kv_kernel(__nv_bfloat16 *q_out, const float *qkv, __nv_bfloat16 *k_cache,
@@ -559,6 +636,33 @@ JL_EXPORT int jl_aux_silu_mul(float *out, void *operand_out, const float *gu, in
     int gx = (ffn / 4 + 255) / 256;
     if (gx > 64) gx = 64;
     return aux_launch(aux_silu_mul_kernel, dim3(gx, n), dim3(256), (cudaStream_t)stream, out, gu, ffn);
+}
+
+JL_EXPORT int jl_aux_silu_mul_gemm(void *rows_f16, float *inv_scale, const float *gu, int n, int ffn, void *stream) {
+    if (!rows_f16 || !inv_scale || !gu || n < 1 || ffn < 256 || ffn % 256) return JL_EINVAL;
+    if (aux_misaligned(rows_f16) || aux_misaligned(gu)) return JL_EINVAL;
+    if (ffn > 50 * 1024) return JL_DECLINED;      // the f32 row does not fit shared memory
+    const int smem = ffn * 4;
+    if (smem > 48 * 1024 - 64 && cudaFuncSetAttribute(aux_silu_mul_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return JL_ECUDA;
+    }
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n); cfg.blockDim = dim3(512); cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)stream; cfg.attrs = at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, aux_silu_mul_gemm_kernel, (__half *)rows_f16, inv_scale, gu, ffn) != cudaSuccess) { cudaGetLastError(); return JL_ECUDA; }
+    return JL_OK;
+}
+
+JL_EXPORT int jl_aux_rope_prefill(void *q_out_bf16, const float *qkv, void *k_cache_bf16, void *v_cache_bf16, const float *cos_t,
+                                  const float *sin_t, int n, int slots, int hq, int hkv, int d, int max_len, void *stream) {
+    if (!q_out_bf16 || !qkv || !k_cache_bf16 || !v_cache_bf16 || !cos_t || !sin_t) return JL_EINVAL;
+    if (n < 1 || n > max_len || slots < 1 || hq < 1 || hkv < 1 || d < 2 || d % 2) return JL_EINVAL;
+    if (((uintptr_t)qkv & 7) || ((uintptr_t)q_out_bf16 & 3) || ((uintptr_t)k_cache_bf16 & 3) || ((uintptr_t)v_cache_bf16 & 3)) return JL_EINVAL;
+    return aux_launch(aux_rope_prefill_kernel, dim3(n), dim3(256), (cudaStream_t)stream, (__nv_bfloat16 *)q_out_bf16, qkv,
+                      (__nv_bfloat16 *)k_cache_bf16, (__nv_bfloat16 *)v_cache_bf16, cos_t, sin_t, slots, hq, hkv, d, max_len);
 }
 
 JL_EXPORT int jl_aux_argmax(long long *out, const float *x, int n, int v, void *stream) {

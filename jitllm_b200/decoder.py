@@ -160,8 +160,63 @@ class Decoder:
                                                is_causal=True, enable_gqa=True)       # query head h uses kv head h // g
             return o[0].transpose(0, 1).reshape(T, -1)
 
-        x = self._layers(self.emb[tokens].float(), pos, attend)
-        return self._argmax(x[-1:])
+        x = self._prefill_chain(tokens)
+        if x is None:
+            x = self._layers(self.emb[tokens].float(), pos, attend)[-1:]
+        return self._argmax(x)
+
+    def _gemm_operand(self, w, n):
+        """(rows, 1/scale) where the GEMM takes n activation rows of weight w from, or None."""
+        import ctypes as C
+        rows, inv = C.c_void_p(), C.c_void_p()
+        if self.dev.lib.jl_gemm_operand(self.dev.ctx, w.handle, n, C.byref(rows), C.byref(inv)) != 0:
+            return None
+        return rows, inv
+
+    def _prefill_chain(self, tokens):
+        """The stack over a prompt with one library kernel between two matmuls: the norm and SiLU*up write the GEMM's
+        activation operand, RoPE fills q and the cache. Returns the last row, or None when a shape has no such form."""
+        torch, c, lib = self.torch, self.cfg, self.dev.lib
+        import torch.nn.functional as F
+        T, d = tokens.shape[0], c.head_dim
+        if T < 9 or T > self.max_len or c.n_layer < 1 or c.hidden % 256 or self.ffn_l % 256 or self.ffn_l > 50 * 1024 or d % 2:
+            return None
+        l0 = self.layers[0]
+        ops = [self._gemm_operand(w, T) for w in (l0["qkv"], l0["gu"], l0["down"])]
+        if None in ops:
+            return None
+        st = torch.cuda.current_stream().cuda_stream
+
+        def ok(rc):
+            if rc != 0:
+                raise RuntimeError(f"jl_aux call failed with status {rc}")
+
+        def mm_prepared(w):
+            out = torch.empty(T, w.nrows, device="cuda", dtype=torch.float32)
+            ok(lib.jl_matmul_dev_prepared(self.dev.ctx, out.data_ptr(), 0, w.handle, T, st))
+            return out
+
+        def norm(delta, op):
+            ok(lib.jl_aux_add_rmsnorm_gemm(x.data_ptr(), delta.data_ptr() if delta is not None else None, self.norm_w.data_ptr(),
+                                           c.eps, op[0], op[1], T, c.hidden, st))
+
+        x = self.emb[tokens].float()
+        q = torch.empty(T, self.hq, d, device="cuda", dtype=torch.bfloat16)
+        delta = None
+        for li, l in enumerate(self.layers):
+            kc, vc = self.k_cache[li], self.v_cache[li]
+            norm(delta, ops[0])
+            qkv = mm_prepared(l["qkv"])
+            ok(lib.jl_aux_rope_prefill(q.data_ptr(), qkv.data_ptr(), kc.data_ptr(), vc.data_ptr(), self.cos.data_ptr(),
+                                       self.sin.data_ptr(), T, kc.shape[0], self.hq, self.hkv, d, self.max_len, st))
+            att = F.scaled_dot_product_attention(q.transpose(0, 1)[None], kc[:1, :, :T], vc[:1, :, :T], is_causal=True, enable_gqa=True)
+            # the attention's bf16 rows are exact in the GEMM's f16 operand: no second (low) half for them
+            delta = self._allreduce(self.mm(l["o"], att[0].transpose(0, 1).reshape(T, -1)))
+            norm(delta, ops[1])
+            gu = mm_prepared(l["gu"])
+            ok(lib.jl_aux_silu_mul_gemm(ops[2][0], ops[2][1], gu.data_ptr(), T, self.ffn_l, st))
+            delta = self._allreduce(mm_prepared(l["down"]))
+        return x[-1:] + delta[-1:]
 
     def decode_step(self, tokens, pos_dev):
         """tokens [B] int64, one per sequence, all at position pos_dev (a 1-element int64 DEVICE tensor,
@@ -196,6 +251,9 @@ class Decoder:
         gemm_prep = (not prep) and c.hidden % 256 == 0 and all(
             lib.jl_gemm_operand(ctx, w.handle, B, C.byref(g_rows), C.byref(g_inv)) == 0 for w in (l0["qkv"], l0["gu"], self.head))
 
+        # SiLU*up likewise, for the down projection
+        down_op = self._gemm_operand(l0["down"], B) if gemm_prep and self.ffn_l % 256 == 0 and self.ffn_l <= 50 * 1024 else None
+
         def mv(w, x_f32):
             if gemm_prep and x_f32 is h:
                 out = torch.empty(B, w.nrows, **f32)
@@ -229,8 +287,15 @@ class Decoder:
             ok(lib.jl_aux_attn_decode(None if prep else att.data_ptr(), op, qb.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                                       pos_dev.data_ptr(), self._att_scratch.data_ptr(), B, self.hq, self.hkv, d, self.max_len, st))
             norm(self._allreduce(mv(l["o"], att)))
-            ok(lib.jl_aux_silu_mul(None if prep else a.data_ptr(), op, mv(l["gu"], h).data_ptr(), B, self.ffn_l, st))
-            norm(self._allreduce(mv(l["down"], a)))             # also the next layer's (or the final) norm
+            gu = mv(l["gu"], h)
+            if down_op is not None:
+                ok(lib.jl_aux_silu_mul_gemm(down_op[0], down_op[1], gu.data_ptr(), B, self.ffn_l, st))
+                down = torch.empty(B, c.hidden, **f32)
+                ok(lib.jl_matmul_dev_prepared(ctx, down.data_ptr(), 0, l["down"].handle, B, st))
+            else:
+                ok(lib.jl_aux_silu_mul(None if prep else a.data_ptr(), op, gu.data_ptr(), B, self.ffn_l, st))
+                down = mv(l["down"], a)
+            norm(self._allreduce(down))                         # also the next layer's (or the final) norm
         logits = self.last_logits = mv(self.head, h)
         if self.world > 1:
             import torch.distributed as dist

@@ -10,6 +10,73 @@ from jitllm_b200 import Q4_K, Device, _lib, synth
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("n,ffn", [(1, 256), (33, 1792), (9, 14336)])
+def test_silu_mul_writes_the_gemm_operand(n, ffn):
+    """Bit for bit what the f32 rows become on their way into the GEMM: the same output either way."""
+    L = _lib.load()
+    rng = synth.rng_for(91 + ffn)
+    ntok = max(n, 9)
+    w = synth.q4k_matrix(rng, 256, ffn)
+    st = torch.cuda.current_stream().cuda_stream
+    with Device(0) as d:
+        d.Reserve(256, ffn, ntok)
+        h = d.Upload(Q4_K, w, 256, ffn)
+        rows, inv = C.c_void_p(), C.c_void_p()
+        assert L.jl_gemm_operand(d.ctx, h.handle, ntok, C.byref(rows), C.byref(inv)) == 0
+        gu = torch.randn(ntok, 2 * ffn, device="cuda") * 3
+        if n == 1:
+            gu[0] = 0                                     # a row of zeros has scale 1
+        f32, ref, got = torch.empty(ntok, ffn, device="cuda"), torch.empty(ntok, 256, device="cuda"), torch.empty(ntok, 256, device="cuda")
+        assert L.jl_aux_silu_mul(f32.data_ptr(), None, gu.data_ptr(), ntok, ffn, st) == 0
+        d.MatMulDev(ref, h, f32, ntok, st)
+        assert L.jl_aux_silu_mul_gemm(rows, inv, gu.data_ptr(), ntok, ffn, st) == 0
+        assert L.jl_matmul_dev_prepared(d.ctx, got.data_ptr(), 0, h.handle, ntok, st) == 0
+        torch.cuda.synchronize()
+        assert d.StatusPoll() and torch.equal(got, ref)
+        assert L.jl_aux_silu_mul_gemm(rows, inv, gu.data_ptr(), 1, 255, st) == _lib.EINVAL
+        assert L.jl_aux_silu_mul_gemm(rows, inv, gu.data_ptr(), 1, 51200 + 256, st) == _lib.DECLINED
+
+
+@pytest.mark.parametrize("n,slots,hq,hkv,d,max_len", [(1, 1, 2, 1, 2, 1), (37, 3, 4, 2, 64, 40), (130, 2, 32, 8, 128, 130)])
+def test_rope_prefill_is_the_single_position_kernel_per_row(n, slots, hq, hkv, d, max_len):
+    L = _lib.load()
+    st = torch.cuda.current_stream().cuda_stream
+    qkv = torch.randn(n, (hq + 2 * hkv) * d, device="cuda")
+    ang = torch.arange(max_len, device="cuda").float()[:, None] * torch.rand(d // 2, device="cuda")
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    bf = dict(device="cuda", dtype=torch.bfloat16)
+    q, kc, vc = torch.empty(n, hq, d, **bf), torch.full((slots, hkv, max_len, d), 7.0, **bf), torch.full((slots, hkv, max_len, d), 7.0, **bf)
+    assert L.jl_aux_rope_prefill(q.data_ptr(), qkv.data_ptr(), kc.data_ptr(), vc.data_ptr(), cos.data_ptr(), sin.data_ptr(), n, slots, hq, hkv,
+                                 d, max_len, st) == 0
+    q1, k1, v1 = torch.empty_like(q), torch.full((1, hkv, max_len, d), 7.0, **bf), torch.full((1, hkv, max_len, d), 7.0, **bf)
+    for r in range(n):
+        pos = torch.tensor([r], device="cuda")
+        assert L.jl_aux_rope_kv(q1[r].data_ptr(), qkv[r].data_ptr(), k1.data_ptr(), v1.data_ptr(), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                                1, hq, hkv, d, max_len, st) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(q, q1) and torch.equal(kc, k1.expand_as(kc)) and torch.equal(vc, v1.expand_as(vc))
+
+
+@pytest.mark.parametrize("T", [9, 17, 130])
+def test_prefill_chain_against_the_plain_stack(T):
+    """The same prompt with and without the chain: bf16 q, k, v and cache in both, so a few bf16 roundings apart."""
+    from jitllm_b200.decoder import Config, Decoder
+    cfg = Config(n_layer=2, hidden=512, n_head=4, n_kv=2, head_dim=128, ffn=1024, vocab=512)
+    with Device(0) as dev:
+        dec = Decoder(dev, cfg, max_batch=3, max_len=136, max_prefill=136, seed=5)
+        toks = torch.randint(0, cfg.vocab, (T,), device="cuda")
+        assert dec._prefill_chain(toks) is not None
+        dec.prefill(toks)
+        got, kc, vc = dec.last_logits.clone(), dec.k_cache.clone(), dec.v_cache.clone()
+        dec._prefill_chain = lambda tokens: None
+        dec.prefill(toks)
+        torch.cuda.synchronize()
+        rel = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm())
+        # two layers, each a bf16 rounding (2^-9) of q, k, v that the other path's f32 sums may take the other way
+        assert rel(got, dec.last_logits) <= 2 * 2.0 ** -9 and rel(kc, dec.k_cache) <= 2.0 ** -9 and rel(vc, dec.v_cache) <= 2.0 ** -9
+        assert dec._gemm_operand(dec.layers[0]["qkv"], 8) is None        # eight tokens: the decode kernels
+
+
 # splits that the K range is cut into where tiles leave SMs idle, element counts that are not a multiple of four, every output type
 @pytest.mark.parametrize("nrows,k,ntok", [(257, 2048, 9), (1023, 4096, 31), (4096, 4096, 64), (3, 512, 17)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16, torch.float16])
