@@ -498,14 +498,43 @@ int jl_gemm_tc5_supported(uint32_t type, int nrows, int k, int ntok) {
 
 static int tc5_pick_nt(int ntok_eff) { return ntok_eff > 128 ? 256 : (ntok_eff > 64 ? 128 : 64); }
 
-// How many CTAs share one tile's K range: only when the tiles alone would leave SMs idle.
-static int tc5_ksplit(int nrows, int ntok_eff, int k, int sms) {
+// How many CTAs share one tile's K range when the tiles alone would leave SMs idle.
+static int tc5_ksplit_few(int nrows, int ntok_eff, int k, int sms) {
     const int nt = tc5_pick_nt(ntok_eff);
     const int units = ((nrows + TC5_ROWS - 1) / TC5_ROWS) * ((ntok_eff + nt - 1) / nt);
     int ks = sms / units;
     if (ks > 8) ks = 8;
     if (ks > k / 256) ks = k / 256;
     return ks < 2 ? 1 : ks;
+}
+
+// The same for any batch. More tiles than SMs run in waves, and a last wave that is nearly empty costs as much as a full one:
+// 192 tiles on 148 SMs (a 4096-row matrix at 1531 f32 tokens) are two waves, 65 % full; as thirds of a tile they are four waves of
+// a third. The split with the least estimated time is taken: waves of (k-blocks + a fill and drain worth five of them), and
+// for the partial planes a write and a read of each (0.86 us a k-block, measured on the 256-wide tile; 4 TB/s through L2)
+// and the sum's launch. A split has to win 5 %.
+static int tc5_ksplit(int nrows, int ntok, int split, int k, int sms) {
+    const int ntok_eff = ntok * (split ? 2 : 1);
+    const int few = tc5_ksplit_few(nrows, ntok_eff, k, sms);
+    if (few > 1 || tc5_pick_nt(ntok_eff) < 256) return few;
+    const int units = ((nrows + TC5_ROWS - 1) / TC5_ROWS) * ((ntok_eff + 255) / 256);
+    double plain = 0, best = 0;
+    int ks = 1;
+    for (int s = 1; s <= 4 && s <= k / 256; s++) {
+        const int waves = (units * s + sms - 1) / sms;
+        double us = waves * ((double)k / 64 / s + 5) * 0.86;
+        if (s > 1) us += 5 + (double)s * ntok * nrows * 8 / 4e6;
+        if (s == 1) plain = best = us;
+        else if (us < 0.95 * plain && us < best) { best = us; ks = s; }
+    }
+    return ks;
+}
+
+// The split a call gets: the one above, or without it where the scratch was sized for less.
+static int tc5_split_for(const jl_ctx *ctx, int nrows, int k, int ntok, int split) {
+    const int sms = ctx ? ctx->sm_count : 148;
+    const int ks = tc5_ksplit(nrows, ntok, split, k, sms), few = tc5_ksplit_few(nrows, ntok * (split ? 2 : 1), k, sms);
+    return ks > few && ctx && ctx->scratch_cap < jl_gemm_tc5_scratch_bytes(nrows, k, ntok, split ? JL_DT_F32 : JL_DT_BF16, sms) ? few : ks;
 }
 
 // Answers for f32 activations (what jl_select is asked about: the decode-side entry points take f32), which
@@ -517,7 +546,7 @@ int jl_gemm_tc5_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, j
     const int ntok_eff = 2 * ntok;
     const int nt = tc5_pick_nt(ntok_eff);
     c.kernel = JL_K_TC5; c.warps = TC5_GEMM_THREADS / 32; c.rows_per_cta = TC5_ROWS;
-    c.split_k = tc5_ksplit(nrows, ntok_eff, k, sms);
+    c.split_k = tc5_split_for(ctx, nrows, k, ntok, 1);
     c.tile_m = TC5_M; c.tile_n = nt; c.tile_k = TC5_KB;
     const int units = ((nrows + TC5_ROWS - 1) / TC5_ROWS) * ((ntok_eff + nt - 1) / nt) * c.split_k;
     c.grid = units < sms ? units : sms;
@@ -526,12 +555,19 @@ int jl_gemm_tc5_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, j
     return JL_OK;
 }
 
-size_t jl_gemm_tc5_scratch_bytes(int nrows, int k, int ntok, int x_dtype, int sms) {
+// What a call wants, and (few) what it cannot do without: jl_reserve and the host calls provide the first, a call that finds
+// only the second runs with fewer splits.
+static size_t tc5_scratch(int nrows, int k, int ntok, int x_dtype, int ks) {
     const int ntok_eff = ntok * (x_dtype == JL_DT_F32 ? 2 : 1);
     size_t b = (((size_t)ntok_eff * k * 2 + 255) & ~(size_t)255) + (((size_t)ntok * 4 + 255) & ~(size_t)255);
-    const int ks = tc5_ksplit(nrows, ntok_eff, k, sms);
     if (ks > 1) b += (size_t)ks * ntok * nrows * 4;
     return b + 256;
+}
+size_t jl_gemm_tc5_scratch_bytes(int nrows, int k, int ntok, int x_dtype, int sms) {
+    return tc5_scratch(nrows, k, ntok, x_dtype, tc5_ksplit(nrows, ntok, x_dtype == JL_DT_F32, k, sms));
+}
+static size_t tc5_scratch_few(int nrows, int k, int ntok, int x_dtype, int sms) {
+    return tc5_scratch(nrows, k, ntok, x_dtype, tc5_ksplit_few(nrows, ntok * (x_dtype == JL_DT_F32 ? 2 : 1), k, sms));
 }
 
 template <int WT, int NT, int SA, int SB>
@@ -555,7 +591,7 @@ static int tc5_launch(jl_ctx *ctx, const CUtensorMap &xmap, const tc5_params &p,
 // [2 tok] = hi, [2 tok + 1] = lo (f16, k each) and one f32 1/scale per token. JL_DECLINED when the scratch is too small.
 int jl_gemm_tc5_operand(jl_ctx *ctx, const jl_weight *w, int ntok, void **rows, float **inv_scale) {
     if (!jl_gemm_tc5_supported(w->type, w->nrows, w->k, ntok)) return JL_DECLINED;
-    if (ctx->scratch_cap < jl_gemm_tc5_scratch_bytes(w->nrows, w->k, ntok, JL_DT_F32, ctx->sm_count)) return JL_DECLINED;
+    if (ctx->scratch_cap < tc5_scratch_few(w->nrows, w->k, ntok, JL_DT_F32, ctx->sm_count)) return JL_DECLINED;
     uint8_t *sp = (uint8_t *)ctx->scratch;
     *rows = sp;
     *inv_scale = (float *)(sp + (((size_t)ntok * 2 * w->k * 2 + 255) & ~(size_t)255));
@@ -573,7 +609,7 @@ int jl_launch_gemm_tc5(jl_ctx *ctx, void *out_dev, int out_dtype, const jl_weigh
     if (prepared) x_dtype = JL_DT_F32;
     const int split = x_dtype == JL_DT_F32 ? 1 : 0;
     const int ntok_eff = ntok * (split ? 2 : 1);
-    const size_t need = jl_gemm_tc5_scratch_bytes(nrows, k, ntok, x_dtype, ctx->sm_count);
+    const size_t need = tc5_scratch_few(nrows, k, ntok, x_dtype, ctx->sm_count);
     if (ctx->scratch_cap < need)
         return jl_set_err(ctx, JL_ENOMEM, "GEMM scratch holds %zu bytes, %d tokens x %d x %d need %zu (jl_reserve sizes it)",
                           ctx->scratch_cap, ntok, nrows, k, need);
@@ -607,7 +643,7 @@ int jl_launch_gemm_tc5(jl_ctx *ctx, void *out_dev, int out_dtype, const jl_weigh
     tc5_params p;
     p.nrows = nrows; p.k = k; p.ntok = ntok; p.ntok_eff = ntok_eff; p.split = split;
     p.row_tiles = (nrows + TC5_ROWS - 1) / TC5_ROWS; p.tok_tiles = (ntok_eff + nt - 1) / nt;
-    p.ksplit = tc5_ksplit(nrows, ntok_eff, k, ctx->sm_count);
+    p.ksplit = tc5_split_for(ctx, nrows, k, ntok, split);
     p.out_dtype = out_dtype; p.out = out_dev; p.partial = partial; p.inv_scale = inv_scale; p.w = wbase; p.status = ctx->dev_status;
     p.w_d = q8 ? reinterpret_cast<const uint16_t *>(w->scales) + (size_t)expert * nrows * w->scale_stride : nullptr;
     p.w_d_stride = w->scale_stride;

@@ -102,6 +102,31 @@ def test_split_sum(orc, nrows, k, ntok, out_dtype):
         assert err <= 2.0 ** -11 + (2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -11 if out_dtype == torch.float16 else 0)
 
 
+def test_wave_split_keeps_to_the_scratch():
+    """192 tiles on 148 SMs are split three ways (two full waves' worth in four of a third) when the scratch has room for the
+    partial planes, and run unsplit when it was sized for less: the same sums to f32 order."""
+    nrows, k, ntok = 4096, 14336, 1500
+    rng = synth.rng_for(97)
+    w, x = synth.q4k_matrix(rng, nrows, k), torch.randn(ntok, k, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for big in (True, False):
+        with Device(0) as d:
+            if big:
+                d.Reserve(nrows, k, ntok)
+            else:                                                      # room for the operand rows only (4 bytes an activation)
+                d.Reserve(256, k, ntok)
+            h = d.Upload(Q4_K, w, nrows, k)
+            outs.append((d.Select(Q4_K, nrows, k, ntok).split_k, torch.empty(ntok, nrows, device="cuda")))
+            d.MatMulDev(outs[-1][1], h, x, ntok, st)
+            torch.cuda.synchronize()
+            assert d.StatusPoll()
+    assert outs[0][0] > 1 and outs[1][0] == 1
+    a, b = outs[0][1].double(), outs[1][1].double()
+    # the tensor core's f32 accumulator truncates: each of the k / 16 additions of a sum can lose one unit (2^-23) of it
+    assert float((a - b).norm() / b.norm()) <= k / 16 * 2.0 ** -23
+
+
 # chunks per CTA from one to eight, a last CTA with part of its chunks, sequences that end in any chunk of it
 @pytest.mark.parametrize("n,hq,hkv,pos,max_len", [(64, 32, 8, 2048, 2056), (64, 32, 8, 700, 2056), (64, 8, 8, 513, 1500), (33, 16, 8, 1000, 1001),
                                                    (64, 64, 8, 15, 600), (20, 32, 8, 511, 512)])
