@@ -166,7 +166,8 @@ int jl_stats_get(jl_ctx *ctx, jl_stats *out);
  * at w stay unchanged until jl_forget covers them. Types: Q4_K, Q8_0, MXFP4 on the tensor-core
  * decode kernels; Q4_0, Q5_0, Q5_1, Q5_K, Q6_K (what real Q4_K_M files mix in,
  * format/quant/dequant.go:85-146,399-470) on the one-warp-per-row kernel, which decodes each weight
- * exactly as quant.Dequant32 does. Any other type is DECLINED. */
+ * exactly as quant.Dequant32 does (Q6_K batches above 8 tokens: the integer tensor cores, closer to exact still).
+ * Any other type is DECLINED. */
 int jl_matvec(jl_ctx *ctx, float *out, uint32_t type, const void *w, size_t w_bytes,
               const float *x, int nrows, int k);
 /* CopyForgetter.Forget (engine/nn/device.go:1570-1581): drop every device copy
@@ -328,6 +329,9 @@ void jl_weight_free(jl_ctx *ctx, jl_weight *w);
 /* x_dev [ntok][k] f32, out_dev [ntok][nrows] f32. ntok = 1 is the decode matvec. */
 int jl_matvec_dev(jl_ctx *ctx, float *out_dev, const jl_weight *w, const float *x_dev, int ntok,
                   void *stream);
+/* Q6_K above 8 tokens keeps its converted activations in a workspace of the context (jl_reserve and the upload size it;
+ * without it the row kernel runs): a call on another stream waits for the one before it. Parallel branches of ONE capture
+ * over one context set JL_FLAG_DECODE_CONCURRENT, which keeps Q6_K on the row kernel. */
 int jl_matmul_dev(jl_ctx *ctx, void *out_dev, int out_dtype, const jl_weight *w, const void *x_dev,
                   int x_dtype, int ntok, void *stream);
 /* desc->gate/up/down are jl_weight* banks; biases and all other pointers are device pointers. */

@@ -61,7 +61,7 @@ JL_EXPORT int jl_open(int device, const jl_opts *opts, jl_ctx **out) {
     c->moe_stage = nullptr; c->moe_stage_cap = 0;
     c->q6k_work = nullptr; c->q6k_cap = 0; c->reserved_k = c->reserved_tok = c->q6k_k = 0;
     c->multi_ready = 0;
-    c->q6k_stream = nullptr; c->q6k_done = nullptr; c->q6k_recorded = false;
+    c->q6k_stream = nullptr; c->q6k_done = nullptr; c->q6k_recorded = c->q6k_captured = false;
     c->x_map = c->o_map = nullptr; c->x_map_cap = c->o_map_cap = 0; c->done_map = nullptr; c->done_seq = 0;
     const int words[4] = {0, (int)c->opts.wait_limit_us, 0, 0};   // code, wait limit, the done kernel's sequence counter, spare
     if (cudaMalloc(&c->dev_status, sizeof words) != cudaSuccess ||
@@ -94,6 +94,7 @@ JL_EXPORT void jl_close(jl_ctx *ctx) {
     if (ctx->o_dev) cudaFree(ctx->o_dev);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->q6k_work) cudaFree(ctx->q6k_work);
+    for (void *p : ctx->q6k_outgrown) cudaFree(p);
     if (ctx->q6k_done) cudaEventDestroy(ctx->q6k_done);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->x_pin) cudaFreeHost(ctx->x_pin);

@@ -387,7 +387,11 @@ int jl_gemm_q6k_reserve(jl_ctx *ctx, int k, int ntok) {
     const size_t need = jl_gemm_q6k_scratch_bytes(k, ntok);
     if (ntok <= 8 || ctx->q6k_cap >= need) return JL_OK;
     JL_CUDA(ctx, cudaDeviceSynchronize());   // an earlier launch may still read the old buffer
-    if (ctx->q6k_work) { cudaFree(ctx->q6k_work); ctx->q6k_work = nullptr; ctx->q6k_cap = 0; }
+    if (ctx->q6k_work) {
+        if (ctx->q6k_captured) ctx->q6k_outgrown.push_back(ctx->q6k_work);     // graphs replay with its address
+        else cudaFree(ctx->q6k_work);
+        ctx->q6k_work = nullptr; ctx->q6k_cap = 0; ctx->q6k_captured = false;
+    }
     if (cudaMalloc(&ctx->q6k_work, need) != cudaSuccess) { cudaGetLastError(); ctx->q6k_work = nullptr; return JL_OK; }
     ctx->q6k_cap = need;
     return JL_OK;
@@ -438,7 +442,8 @@ int jl_launch_gemm_q6k(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expe
     // so with JL_FLAG_DECODE_CONCURRENT, which keeps Q6_K on the row kernel (no workspace).
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     JL_CUDA(ctx, cudaStreamIsCapturing(s, &cap));
-    if (cap == cudaStreamCaptureStatusNone) {
+    if (cap != cudaStreamCaptureStatusNone) ctx->q6k_captured = true;
+    else {
         if (!ctx->q6k_done) JL_CUDA(ctx, cudaEventCreateWithFlags(&ctx->q6k_done, cudaEventDisableTiming));
         if (ctx->q6k_recorded && ctx->q6k_stream != s) JL_CUDA(ctx, cudaStreamWaitEvent(s, ctx->q6k_done, 0));
     }

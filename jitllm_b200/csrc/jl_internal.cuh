@@ -121,6 +121,8 @@ struct jl_ctx {
     void *q6k_work; size_t q6k_cap;
     int reserved_k, reserved_tok, q6k_k;
     cudaStream_t q6k_stream; cudaEvent_t q6k_done; bool q6k_recorded;
+    bool q6k_captured;                  // a capture has taken the workspace's address: an outgrown one is kept until jl_close
+    std::vector<void *> q6k_outgrown;
     void *x_pin; size_t x_pin_cap;
     void *o_pin; size_t o_pin_cap;
     int *dev_status;        // device words: [0] code a kernel sets when a bounded wait ran out, [1] the limit (us)

@@ -46,6 +46,36 @@ def test_batch_kernel_matches_float64(orc, nrows, k, ntok):
     print(f"{nrows}x{k} {ntok} tokens: batch kernel {rel(got, ref):.2e}, row kernel {simt:.2e}")
 
 
+def test_batch_kernel_in_a_graph_and_on_two_streams(orc):
+    """A captured call keeps its workspace when a later reserve outgrows it; calls on two streams share it in order."""
+    rng = synth.rng_for(80)
+    nrows, k, ntok = 256, 1024, 20
+    w, xs = synth.matrix(rng, Q6_K, nrows, k), [torch.from_numpy(synth.activations(rng, ntok, k)).cuda() for _ in range(2)]
+    with Device(0) as dev:
+        dev.Reserve(nrows, k, ntok)
+        h = dev.Upload(Q6_K, w, nrows, k)
+        outs = [torch.empty(ntok, nrows, device="cuda") for _ in range(3)]
+        ss = [torch.cuda.Stream(), torch.cuda.Stream()]
+        torch.cuda.synchronize()
+        for _ in range(20):
+            for i in range(2):
+                dev.MatMulDev(outs[i], h, xs[i], ntok, ss[i].cuda_stream)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=ss[0]):
+            dev.MatMulDev(outs[2], h, xs[1], ntok, ss[0].cuda_stream)
+        dev.Reserve(4096, 4096, 300)
+        other = torch.empty(300, nrows, device="cuda")
+        dev.MatMulDev(other, h, torch.randn(300, k, device="cuda"), 300, ss[1].cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        assert dev.StatusPoll() and torch.equal(outs[2], outs[1])
+        for o, x in zip(outs, xs):
+            ref = orc.matmul_f64(Q6_K, w, x.cpu().numpy(), nrows, k, ntok)
+            assert rel(o.cpu().numpy(), ref) <= (4 + k / 256 / 2) * 2.0 ** -24
+        h.free()
+
+
 @pytest.mark.parametrize("dist", ["one_huge", "tiny", "huge", "zeros"])
 def test_batch_kernel_input_distributions(orc, dist):
     rng = synth.rng_for(78)
