@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const uint8_t *__restric
             }
         } else if (jl_type_raw_simt(TYPE)) {
             // raw ggml blocks; each weight exactly as quant.Dequant32 forms it
-            constexpr int BE = TYPE == JL_TYPE_Q5_K || TYPE == JL_TYPE_Q6_K ? 256 : 32;
-            constexpr int BB = TYPE == JL_TYPE_Q4_0 ? 18 : TYPE == JL_TYPE_Q5_0 ? 22 : TYPE == JL_TYPE_Q5_1 ? 24 : TYPE == JL_TYPE_Q5_K ? 176 : 210;
+            constexpr int BE = TYPE == JL_TYPE_Q5_K ? 256 : 32;
+            constexpr int BB = TYPE == JL_TYPE_Q4_0 ? 18 : TYPE == JL_TYPE_Q5_0 ? 22 : TYPE == JL_TYPE_Q5_1 ? 24 : 176;
             const uint8_t *blk = data + ((size_t)row * (k / BE) + (size_t)(si * 32 / BE)) * BB;
             const int e0 = (si * 32) % BE;
             for (int l = 0; l < 32; l++) acc = fmaf(jl_raw_weight(TYPE, blk, e0 + l), xs[l], acc);

@@ -58,7 +58,8 @@ __host__ __device__ static inline void jl_raw_record(uint32_t t, const uint8_t *
 }
 
 #ifdef __CUDACC__
-// The f32 weight of element e, rounded where quant.Dequant32 rounds.
+// The f32 weight of element e, rounded where quant.Dequant32 rounds (Q6_K, whose resident blocks lack their d, has kernels of its
+// own).
 __device__ static inline float jl_raw_weight(uint32_t t, const uint8_t *blk, int e) {
     const int q = jl_raw_code(t, blk, e);
     switch (t) {
@@ -73,12 +74,6 @@ __device__ static inline float jl_raw_weight(uint32_t t, const uint8_t *blk, int
         jl_raw_scale_min_k4(e >> 5, blk + 4, &sc, &m);
         const float d = __half2float(__ushort_as_half(jl_raw_le16(blk))), dmin = __half2float(__ushort_as_half(jl_raw_le16(blk + 2)));
         return __fsub_rn(__fmul_rn(__fmul_rn(d, (float)sc), (float)q), __fmul_rn(dmin, (float)m));
-    }
-    case JL_TYPE_Q6_K: {  // (d sc) (q - 32), sc the int8 scale of the element's 16-run
-        const float d = __half2float(__ushort_as_half(jl_raw_le16(blk + 208)));
-        const int n = e >> 7, j = (e >> 5) & 3, l = e & 31;
-        const int sc = (int)(int8_t)blk[192 + n * 8 + (l >> 4) + 2 * j];
-        return __fmul_rn(__fmul_rn(d, (float)sc), (float)(q - 32));
     }
     }
     return 0.f;
