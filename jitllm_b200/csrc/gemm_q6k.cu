@@ -2,7 +2,7 @@
 //
 // A Q6_K weight is d * sc * (q - 32): an integer w = sc (q - 32) of at most 13 bits times the super-block's f16 d. The row
 // kernel serves it with f32 weights and f32 activations, and at 203 tokens of 4096 x 14336 that is 3.4 ms of FP32 FMAs
-// (7 TFLOP/s); this kernel takes 154 us (155 TFLOP/s), activation planes included. Both sides are integers and nothing
+// (7 TFLOP/s); this kernel takes 141 us (169 TFLOP/s), activation planes included. Both sides are integers and nothing
 // is rounded inside a super-block:
 //
 //   weights      w = 256 h + l, both signed bytes (|w| <= 4096): two int8 operands.
@@ -17,7 +17,7 @@
 //                them, times d and 1/scale, to the token's f32 accumulator in registers. 56 such additions per output
 //                at k = 14336, where the row kernel makes one per element.
 //
-// Work split: a CTA is 128 rows x T tokens (T = 16, 32 or 64) x a slice of the super-blocks; the slices of a tile are the
+// Work split: a CTA is 128 rows x T tokens (T = 16, 24 .. 64) x a slice of the super-blocks; the slices of a tile are the
 // CTAs of one thread-block cluster, which add their f32 tiles in rank order through distributed shared memory (bit-stable;
 // nothing is waited for but the cluster barrier). Roles: warps 0..3 drain, warp 4 copies the activation planes (untiled bulk
 // copies: the prep kernel writes them as the swizzled shared-memory image), warp 5 issues the MMAs, warps 6..13 make the
@@ -43,7 +43,7 @@ q6k_xprep_kernel(const float *__restrict__ X, uint8_t *__restrict__ planes, floa
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int lane = threadIdx.x & 31, sb = blockIdx.x;
-    const int tok = blockIdx.y * 8 + (threadIdx.x >> 5);         // the padded token count is a multiple of 16
+    const int tok = blockIdx.y * 8 + (threadIdx.x >> 5);         // the padded token count is a multiple of 8
     const int tt = tok / T, t = tok - tt * T;
     float v[8];
     uint32_t amax = 0;
@@ -99,7 +99,8 @@ struct q6g_smem {
     static constexpr int INV_OFS = BAR_OFS + (2 * Q6G_STAGES + 4) * 8; // [4 warps][T] 1 / scale of the drained super-block
     static constexpr int MISC_OFS = INV_OFS + 4 * T * 4;
     static constexpr int TOTAL = MISC_OFS + 16 + 1024;
-    static constexpr int COLS = 8 * T;                                 // two accumulators of 4 T columns
+    static constexpr int COLS = T <= 16 ? 128 : (T <= 32 ? 256 : 512); // two accumulators of 4 T columns, a power of two allocated
+    static_assert(T % 8 == 0 && STAGE % 1024 == 0, "operands start on swizzle atoms");
 };
 
 __device__ __forceinline__ void q6g_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -364,8 +365,13 @@ __global__ void __launch_bounds__(Q6G_THREADS, 1) gemm_q6k_kernel(const q6g_para
 
 // ------------------------------------------------------------------------- host
 
-// Tokens of a tile: the smallest that covers the batch, 64 at most (8 T columns are all of TMEM at 64).
-static int q6g_tile(int ntok) { return ntok <= 16 ? 16 : (ntok <= 32 ? 32 : 64); }
+// Tokens of a tile: the batch over the fewest tiles of 64 (8 T columns are all of TMEM there), rounded up to 8. The MMAs
+// are what bounds the kernel and their N is 4 T: 203 tokens of 4096 x 14336 as four tiles of 64 took 154 us, of 56 take 141; 140
+// tokens as three of 64 153, of 48 124.
+static int q6g_tile(int ntok) {
+    const int tiles = (ntok + 63) / 64, T = ((ntok + tiles - 1) / tiles + 7) & ~7;
+    return T < 16 ? 16 : T;
+}
 
 // CTAs that share a tile's super-blocks: only as many as fill SMs that the tiles alone would leave idle.
 static int q6g_slices(int nrows, int nsb, int ntok, int sms) {
@@ -464,7 +470,16 @@ int jl_launch_gemm_q6k(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expe
     cfg.attrs = at; cfg.numAttrs = (ctx->opts.flags & JL_FLAG_NO_PDL) ? 0 : 1;
     JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, q6k_xprep_kernel, x_dev, planes, inv, nsb, ntok, T));
     ctx->st.launches++;
-    const int rc = T == 16 ? q6g_launch<16>(ctx, p, tok_tiles, s) : T == 32 ? q6g_launch<32>(ctx, p, tok_tiles, s) : q6g_launch<64>(ctx, p, tok_tiles, s);
+    int rc;
+    switch (T) {
+    case 16: rc = q6g_launch<16>(ctx, p, tok_tiles, s); break;
+    case 24: rc = q6g_launch<24>(ctx, p, tok_tiles, s); break;
+    case 32: rc = q6g_launch<32>(ctx, p, tok_tiles, s); break;
+    case 40: rc = q6g_launch<40>(ctx, p, tok_tiles, s); break;
+    case 48: rc = q6g_launch<48>(ctx, p, tok_tiles, s); break;
+    case 56: rc = q6g_launch<56>(ctx, p, tok_tiles, s); break;
+    default: rc = q6g_launch<64>(ctx, p, tok_tiles, s); break;
+    }
     if (rc == JL_OK && cap == cudaStreamCaptureStatusNone) {
         JL_CUDA(ctx, cudaEventRecord(ctx->q6k_done, s));
         ctx->q6k_stream = s;

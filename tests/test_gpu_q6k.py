@@ -25,7 +25,7 @@ def run(dev, w, nrows, k, x):
     return out.cpu().numpy()
 
 
-# one super-block and one row, tile edges (128 rows; 16, 32, 64 tokens), every number of k slices, odd rows and tokens
+# one super-block and one row, tile edges (128 rows; every tile of 16 to 64 tokens), every number of k slices, odd rows and tokens
 @pytest.mark.parametrize("nrows,k,ntok", [(1, 256, 9), (37, 512, 16), (128, 768, 17), (129, 1024, 32), (300, 2048, 33), (256, 1280, 64),
                                           (511, 3584, 65), (4096, 4096, 203), (16384, 512, 64), (1024, 14336, 130)])
 def test_batch_kernel_matches_float64(orc, nrows, k, ntok):
