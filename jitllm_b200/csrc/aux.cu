@@ -167,6 +167,13 @@ __global__ void __launch_bounds__(256) aux_add_rmsnorm_gemm_kernel(float *x_io, 
         }
 }
 
+// SiLU(g) * u with expf, whose error does not grow with the exponent: __expf put 7 units of the last place into elements whose
+// gate is far below zero (worst of 900,000: 8.8e-7 relative, now under 3e-7). The callers are bound by memory.
+__device__ __forceinline__ float aux_silu_mul1(float g, float u) { return g / (1.f + expf(-g)) * u; }
+__device__ __forceinline__ float4 aux_silu_mul4(const float4 &g, const float4 &u) {
+    return make_float4(aux_silu_mul1(g.x, u.x), aux_silu_mul1(g.y, u.y), aux_silu_mul1(g.z, u.z), aux_silu_mul1(g.w, u.w));
+}
+
 // One warp per 256 outputs: out and/or the prepared operand of the matvec that consumes them.
 __global__ void __launch_bounds__(128) aux_silu_mul_sb_kernel(float *out, uint8_t *operand, const float *gu, int ffn) {
     AUX_PDL();
@@ -179,8 +186,7 @@ __global__ void __launch_bounds__(128) aux_silu_mul_sb_kernel(float *out, uint8_
     for (int hf = 0; hf < 2; ++hf) {
         const int i = sb * 64 + hf * 32 + lane;
         const float4 g = g4[i], u = u4[i];
-        v[hf] = make_float4(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y,
-                            g.z / (1.f + __expf(-g.z)) * u.z, g.w / (1.f + __expf(-g.w)) * u.w);
+        v[hf] = aux_silu_mul4(g, u);
         if (out) ((float4 *)(out + (size_t)row * ffn))[i] = v[hf];
     }
     if (operand) q4k_prep_sb_vals(v[0], v[1], operand + ((size_t)row * nsb + sb) * Q4K_XP_SB_BYTES, lane);
@@ -193,8 +199,7 @@ __global__ void __launch_bounds__(256) aux_silu_mul_kernel(float *out, const flo
     float4 *o4 = (float4 *)(out + (size_t)blockIdx.y * ffn);
     for (int i = blockIdx.x * 256 + threadIdx.x; i < ffn / 4; i += gridDim.x * 256) {
         float4 g = g4[i], u = u4[i];
-        o4[i] = make_float4(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y,
-                            g.z / (1.f + __expf(-g.z)) * u.z, g.w / (1.f + __expf(-g.w)) * u.w);
+        o4[i] = aux_silu_mul4(g, u);
     }
 }
 
@@ -211,8 +216,7 @@ __global__ void __launch_bounds__(512) aux_silu_mul_gemm_kernel(__half *rows, fl
     float amax = 0.f;
     for (int i = threadIdx.x; i < ffn / 4; i += 512) {
         const float4 g = g4[i], u = u4[i];
-        const float4 v = make_float4(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y,
-                                     g.z / (1.f + __expf(-g.z)) * u.z, g.w / (1.f + __expf(-g.w)) * u.w);
+        const float4 v = aux_silu_mul4(g, u);
         srow[i] = v;
         amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }

@@ -37,6 +37,19 @@ def test_silu_mul_writes_the_gemm_operand(n, ffn):
         assert L.jl_aux_silu_mul_gemm(rows, inv, gu.data_ptr(), 1, 51200 + 256, st) == _lib.DECLINED
 
 
+# a width of whole super-blocks (the form the operands share) and one that is not
+@pytest.mark.parametrize("ffn", [14336, 1000])
+def test_silu_mul_rounds_like_f32(ffn):
+    """expf (2 units of the last place at most), 1 + e, the quotient and the product: 2 + 3/2 units of 2^-23 and their mixed terms."""
+    L = _lib.load()
+    gu = torch.randn(64, 2 * ffn, device="cuda") * 4
+    gu[0, :ffn] = torch.linspace(-80, 80, ffn, device="cuda")
+    out = torch.empty(64, ffn, device="cuda")
+    assert L.jl_aux_silu_mul(out.data_ptr(), None, gu.data_ptr(), 64, ffn, torch.cuda.current_stream().cuda_stream) == 0
+    ref = torch.nn.functional.silu(gu[:, :ffn].double()) * gu[:, ffn:].double()
+    assert float(((out.double() - ref).abs() / ref.abs()).max()) <= 3.6 * 2.0 ** -23
+
+
 @pytest.mark.parametrize("n,slots,hq,hkv,d,max_len", [(1, 1, 2, 1, 2, 1), (37, 3, 4, 2, 64, 40), (130, 2, 32, 8, 128, 130)])
 def test_rope_prefill_is_the_single_position_kernel_per_row(n, slots, hq, hkv, d, max_len):
     L = _lib.load()
