@@ -173,17 +173,29 @@ class Decoder:
             return None
         return rows, inv
 
+    def _gemm_operands(self, n):
+        """weight -> its operand for n rows or None, asked once per type and shape: a stack may mix formats (a file that keeps half
+        of its down and v matrices in Q6_K), and only some of them take a prepared operand."""
+        known = {}
+
+        def of(w):
+            key = (w.type, w.nrows, w.k)
+            if key not in known:
+                known[key] = self._gemm_operand(w, n) if w.k % 256 == 0 else None
+            return known[key]
+        return of
+
     def _prefill_chain(self, tokens):
         """The stack over a prompt with one library kernel between two matmuls: the norm and SiLU*up write the GEMM's
-        activation operand, RoPE fills q and the cache. Returns the last row, or None when a shape has no such form."""
+        activation operand where the next matrix takes one (f32 rows otherwise), RoPE fills q and the cache. Returns the last
+        row, or None when a shape has no such form."""
         torch, c, lib = self.torch, self.cfg, self.dev.lib
         import torch.nn.functional as F
         T, d = tokens.shape[0], c.head_dim
         if T < 9 or T > self.max_len or c.n_layer < 1 or c.hidden % 256 or self.ffn_l % 256 or self.ffn_l > 50 * 1024 or d % 2:
             return None
-        l0 = self.layers[0]
-        ops = [self._gemm_operand(w, T) for w in (l0["qkv"], l0["gu"], l0["down"])]
-        if None in ops:
+        op = self._gemm_operands(T)
+        if all(op(l[name]) is None for l in self.layers for name in ("qkv", "gu", "down")):
             return None
         st = torch.cuda.current_stream().cuda_stream
 
@@ -196,26 +208,36 @@ class Decoder:
             ok(lib.jl_matmul_dev_prepared(self.dev.ctx, out.data_ptr(), 0, w.handle, T, st))
             return out
 
-        def norm(delta, op):
-            ok(lib.jl_aux_add_rmsnorm_gemm(x.data_ptr(), delta.data_ptr() if delta is not None else None, self.norm_w.data_ptr(),
-                                           c.eps, op[0], op[1], T, c.hidden, st))
+        def norm_mm(delta, w):
+            dp = delta.data_ptr() if delta is not None else None
+            if op(w) is not None:
+                ok(lib.jl_aux_add_rmsnorm_gemm(x.data_ptr(), dp, self.norm_w.data_ptr(), c.eps, *op(w), T, c.hidden, st))
+                return mm_prepared(w)
+            h = torch.empty_like(x)
+            ok(lib.jl_aux_add_rmsnorm(x.data_ptr(), dp, self.norm_w.data_ptr(), c.eps, h.data_ptr(), None, T, c.hidden, st))
+            return self.mm(w, h)
 
         x = self.emb[tokens].float()
         q = torch.empty(T, self.hq, d, device="cuda", dtype=torch.bfloat16)
         delta = None
         for li, l in enumerate(self.layers):
             kc, vc = self.k_cache[li], self.v_cache[li]
-            norm(delta, ops[0])
-            qkv = mm_prepared(l["qkv"])
+            qkv = norm_mm(delta, l["qkv"])
             ok(lib.jl_aux_rope_prefill(q.data_ptr(), qkv.data_ptr(), kc.data_ptr(), vc.data_ptr(), self.cos.data_ptr(),
                                        self.sin.data_ptr(), T, kc.shape[0], self.hq, self.hkv, d, self.max_len, st))
             att = F.scaled_dot_product_attention(q.transpose(0, 1)[None], kc[:1, :, :T], vc[:1, :, :T], is_causal=True, enable_gqa=True)
-            # the attention's bf16 rows are exact in the GEMM's f16 operand: no second (low) half for them
-            delta = self._allreduce(self.mm(l["o"], att[0].transpose(0, 1).reshape(T, -1)))
-            norm(delta, ops[1])
-            gu = mm_prepared(l["gu"])
-            ok(lib.jl_aux_silu_mul_gemm(ops[2][0], ops[2][1], gu.data_ptr(), T, self.ffn_l, st))
-            delta = self._allreduce(mm_prepared(l["down"]))
+            att = att[0].transpose(0, 1).reshape(T, -1)
+            # the GEMM takes the attention's bf16 rows as they are (each is its own high half: the low half of the f32 form is
+            # zero); the row kernels take f32
+            delta = self._allreduce(self.mm(l["o"], att if op(l["o"]) is not None else att.float()))
+            gu = norm_mm(delta, l["gu"])
+            if op(l["down"]) is not None:
+                ok(lib.jl_aux_silu_mul_gemm(*op(l["down"]), gu.data_ptr(), T, self.ffn_l, st))
+                delta = self._allreduce(mm_prepared(l["down"]))
+            else:
+                a = torch.empty(T, self.ffn_l, device="cuda", dtype=torch.float32)
+                ok(lib.jl_aux_silu_mul(a.data_ptr(), None, gu.data_ptr(), T, self.ffn_l, st))
+                delta = self._allreduce(self.mm(l["down"], a))
         return x[-1:] + delta[-1:]
 
     def decode_step(self, tokens, pos_dev):
@@ -236,67 +258,63 @@ class Decoder:
                 raise RuntimeError(f"jl_aux call failed with status {rc}")
 
         ctx = self.dev.ctx
-        l0 = self.layers[0]
-        # With few sequences every producer writes the next matvec's prepared activation operand itself
-        # (no conversion launch in between); otherwise f32 rows go to the GEMM path.
-        ops = [lib.jl_decode_operand(ctx, w.handle, B) for w in (l0["qkv"], l0["o"], l0["gu"], l0["down"], self.head)]
+        # With few sequences every producer writes the next matvec's prepared activation operand itself (no conversion launch in
+        # between), where every matrix of the stack takes one; otherwise f32 rows.
+        ops = []
+        if B <= 8:
+            shapes = {(w.type, w.nrows, w.k): w for l in self.layers + [dict(head=self.head)] for w in l.values()}
+            ops = [lib.jl_decode_operand(ctx, w.handle, B) for w in shapes.values()]
         prep = B <= 8 and all(ops) and (self.hq // self.hkv) % 2 == 0
         op = ops[0] if prep else None
 
-        # With many sequences the norm writes the tcgen05 GEMM's activation operand (f16 hi / lo rows + per-row scale)
-        # for its consumers (q|k|v, gate|up, the head: all of width hidden, so one place serves the three), again with
-        # no conversion launch in between.
-        import ctypes as C
-        g_rows, g_inv = C.c_void_p(), C.c_void_p()
-        gemm_prep = (not prep) and c.hidden % 256 == 0 and all(
-            lib.jl_gemm_operand(ctx, w.handle, B, C.byref(g_rows), C.byref(g_inv)) == 0 for w in (l0["qkv"], l0["gu"], self.head))
+        # With many sequences the norm and SiLU*up write the tcgen05 GEMM's activation operand (f16 hi / lo rows + per-row
+        # scale) for the matrices that take one, again with no conversion launch in between.
+        operands = self._gemm_operands(B)
+        gemm_op = lambda w: None if prep else operands(w)
 
-        # SiLU*up likewise, for the down projection
-        down_op = self._gemm_operand(l0["down"], B) if gemm_prep and self.ffn_l % 256 == 0 and self.ffn_l <= 50 * 1024 else None
+        def mm_prepared(w):
+            out = torch.empty(B, w.nrows, **f32)
+            ok(lib.jl_matmul_dev_prepared(ctx, out.data_ptr(), 0, w.handle, B, st))         # 0 = JL_DT_F32
+            return out
 
         def mv(w, x_f32):
-            if gemm_prep and x_f32 is h:
-                out = torch.empty(B, w.nrows, **f32)
-                ok(lib.jl_matmul_dev_prepared(ctx, out.data_ptr(), 0, w.handle, B, st))     # 0 = JL_DT_F32
-                return out
             if not prep:
                 return self.mm(w, x_f32)
             out = torch.empty(B, w.nrows, **f32)
             ok(lib.jl_matvec_dev_prepared(ctx, out.data_ptr(), w.handle, B, st))
             return out
 
-        def norm(delta):
-            if gemm_prep:
-                ok(lib.jl_aux_add_rmsnorm_gemm(x.data_ptr(), delta.data_ptr() if delta is not None else None,
-                                               self.norm_w.data_ptr(), c.eps, g_rows, g_inv, B, c.hidden, st))
-                return
-            ok(lib.jl_aux_add_rmsnorm(x.data_ptr(), delta.data_ptr() if delta is not None else None, self.norm_w.data_ptr(),
-                                      c.eps, None if prep else h.data_ptr(), op, B, c.hidden, st))
+        def norm_mv(delta, w):
+            dp, g = delta.data_ptr() if delta is not None else None, gemm_op(w)
+            if g is not None:
+                ok(lib.jl_aux_add_rmsnorm_gemm(x.data_ptr(), dp, self.norm_w.data_ptr(), c.eps, *g, B, c.hidden, st))
+                return mm_prepared(w)
+            ok(lib.jl_aux_add_rmsnorm(x.data_ptr(), dp, self.norm_w.data_ptr(), c.eps, None if prep else h.data_ptr(), op, B, c.hidden, st))
+            return mv(w, h)
 
         x = self.emb[tokens].float()
         h = torch.empty_like(x)
         qb = torch.empty(B, self.hq, d, device="cuda", dtype=torch.bfloat16)
         att = torch.empty(B, self.hq * d, **f32)
         a = torch.empty(B, self.ffn_l, **f32)
-        norm(None)
+        delta = None
         for li, l in enumerate(self.layers):
-            qkv = mv(l["qkv"], h)
+            qkv = norm_mv(delta, l["qkv"])
             kc, vc = self.k_cache[li], self.v_cache[li]
             ok(lib.jl_aux_rope_kv(qb.data_ptr(), qkv.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos_dev.data_ptr(),
                                   self.cos.data_ptr(), self.sin.data_ptr(), B, self.hq, self.hkv, d, self.max_len, st))
             ok(lib.jl_aux_attn_decode(None if prep else att.data_ptr(), op, qb.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                                       pos_dev.data_ptr(), self._att_scratch.data_ptr(), B, self.hq, self.hkv, d, self.max_len, st))
-            norm(self._allreduce(mv(l["o"], att)))
-            gu = mv(l["gu"], h)
-            if down_op is not None:
-                ok(lib.jl_aux_silu_mul_gemm(down_op[0], down_op[1], gu.data_ptr(), B, self.ffn_l, st))
-                down = torch.empty(B, c.hidden, **f32)
-                ok(lib.jl_matmul_dev_prepared(ctx, down.data_ptr(), 0, l["down"].handle, B, st))
+            gu = norm_mv(self._allreduce(mv(l["o"], att)), l["gu"])
+            g = gemm_op(l["down"]) if self.ffn_l <= 50 * 1024 else None
+            if g is not None:
+                ok(lib.jl_aux_silu_mul_gemm(*g, gu.data_ptr(), B, self.ffn_l, st))
+                down = mm_prepared(l["down"])
             else:
                 ok(lib.jl_aux_silu_mul(None if prep else a.data_ptr(), op, gu.data_ptr(), B, self.ffn_l, st))
                 down = mv(l["down"], a)
-            norm(self._allreduce(down))                         # also the next layer's (or the final) norm
-        logits = self.last_logits = mv(self.head, h)
+            delta = self._allreduce(down)
+        logits = self.last_logits = norm_mv(delta, self.head)
         if self.world > 1:
             import torch.distributed as dist
             parts = [torch.empty_like(logits) for _ in range(self.world)]

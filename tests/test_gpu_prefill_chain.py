@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from jitllm_b200 import Q4_K, Device, _lib, synth
+from jitllm_b200 import Q4_K, Q6_K, Device, _lib, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -88,6 +88,38 @@ def test_prefill_chain_against_the_plain_stack(T):
         # two layers, each a bf16 rounding (2^-9) of q, k, v that the other path's f32 sums may take the other way
         assert rel(got, dec.last_logits) <= 2 * 2.0 ** -9 and rel(kc, dec.k_cache) <= 2.0 ** -9 and rel(vc, dec.v_cache) <= 2.0 ** -9
         assert dec._gemm_operand(dec.layers[0]["qkv"], 8) is None        # eight tokens: the decode kernels
+
+
+@pytest.mark.parametrize("name,rows,k", [("qkv", 1024, 512), ("o", 512, 512), ("gu", 2048, 512), ("down", 512, 1024), ("head", 512, 512)])
+@pytest.mark.parametrize("layer", [0, 1])
+def test_a_stack_of_mixed_formats(name, rows, k, layer):
+    """One Q6_K matrix in a Q4_K stack, in any layer: a prompt, a batched step and a small batch's step run, and agree with
+    the plain stack."""
+    from jitllm_b200.decoder import Config, Decoder
+    cfg = Config(n_layer=2, hidden=512, n_head=4, n_kv=2, head_dim=128, ffn=1024, vocab=512)
+    rel = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm())
+    # three bf16 roundings (2^-9 each) of q, k, v and the attention's rows that the other path's f32 sums may take the other way
+    bar = 3 * 2.0 ** -9
+    with Device(0) as dev:
+        dec = Decoder(dev, cfg, max_batch=12, max_len=64, max_prefill=40, seed=5)
+        w = dev.Upload(Q6_K, synth.matrix(synth.rng_for(6), Q6_K, rows, k), rows, k)
+        if name == "head":
+            dec.head = w
+        else:
+            dec.layers[layer][name] = w
+        toks = torch.randint(0, cfg.vocab, (40,), device="cuda")
+        dec.prefill(toks)
+        got, kc, vc = dec.last_logits.clone(), dec.k_cache.clone(), dec.v_cache.clone()
+        chain, dec._prefill_chain = dec._prefill_chain, lambda tokens: None
+        dec.prefill(toks)
+        assert rel(got, dec.last_logits) <= bar and rel(kc, dec.k_cache) <= bar and rel(vc, dec.v_cache) <= bar
+        for B in (12, 4):
+            pos = torch.tensor([40], device="cuda")
+            dec.decode_step_torch(toks[:B], pos)
+            ref = dec.last_logits.clone()
+            dec.decode_step(toks[:B], pos)
+            torch.cuda.synchronize()
+            assert dev.StatusPoll() and rel(dec.last_logits, ref) <= bar
 
 
 # splits that the K range is cut into where tiles leave SMs idle, element counts that are not a multiple of four, every output type
