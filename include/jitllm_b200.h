@@ -326,7 +326,10 @@ int jl_weight_upload(jl_ctx *ctx, uint32_t type, const void *w_host, size_t w_by
 int jl_weight_upload_bank(jl_ctx *ctx, uint32_t type, const void *w_host, size_t w_bytes,
                           int n_expert, int nrows, int k, jl_weight **out);
 void jl_weight_free(jl_ctx *ctx, jl_weight *w);
-/* x_dev [ntok][k] f32, out_dev [ntok][nrows] f32. ntok = 1 is the decode matvec. */
+/* x_dev [ntok][k] f32, out_dev [ntok][nrows] f32. ntok = 1 is the decode matvec.
+ * Q4_K calls of 2 to 8 tokens that convert x first hold it in a place that belongs to their stream: the first eight streams of
+ * a context have one, a captured call takes memory of its graph's own (allocated at the capture, given back once the graph
+ * is gone), and a call without a place runs on a form that reads x itself. Such calls need no order among streams and graphs. */
 int jl_matvec_dev(jl_ctx *ctx, float *out_dev, const jl_weight *w, const float *x_dev, int ntok,
                   void *stream);
 /* Q6_K above 8 tokens keeps its converted activations in a workspace of the context (jl_reserve and the upload size it;

@@ -61,6 +61,7 @@ JL_EXPORT int jl_open(int device, const jl_opts *opts, jl_ctx **out) {
     c->moe_stage = nullptr; c->moe_stage_cap = 0;
     c->q6k_work = nullptr; c->q6k_cap = 0; c->reserved_k = c->reserved_tok = c->q6k_k = 0;
     c->multi_ready = 0;
+    c->xop = nullptr; c->xop_slot = 0; c->xop_streams = 0;
     c->q6k_stream = nullptr; c->q6k_done = nullptr; c->q6k_recorded = c->q6k_captured = false;
     c->x_map = c->o_map = nullptr; c->x_map_cap = c->o_map_cap = 0; c->done_map = nullptr; c->done_seq = 0;
     const int words[4] = {0, (int)c->opts.wait_limit_us, 0, 0};   // code, wait limit, the done kernel's sequence counter, spare
@@ -93,6 +94,8 @@ JL_EXPORT void jl_close(jl_ctx *ctx) {
     if (ctx->x_dev) cudaFree(ctx->x_dev);
     if (ctx->o_dev) cudaFree(ctx->o_dev);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->xop) cudaFree(ctx->xop);
+    jl_places_free(ctx, true);
     if (ctx->q6k_work) cudaFree(ctx->q6k_work);
     for (void *p : ctx->q6k_outgrown) cudaFree(p);
     if (ctx->q6k_done) cudaEventDestroy(ctx->q6k_done);
@@ -190,8 +193,10 @@ JL_EXPORT int jl_reserve(jl_ctx *ctx, int max_rows, int max_k, int max_tok) {
         if (rows == max_rows) break;
     }
     if (max_tok > 8 && need_gemm > need) need = need_gemm;
+    jl_places_free(ctx, false);
     int rc = jl_grow_scratch(ctx, need);
     if (rc) return rc;
+    if ((rc = jl_xop_reserve(ctx, jl_gemv_scratch_bytes(JL_TYPE_Q4_K, k256, dtok)))) return rc;
     if (k256 > ctx->reserved_k) ctx->reserved_k = k256;
     if (max_tok > ctx->reserved_tok) ctx->reserved_tok = max_tok;
     if (ctx->q6k_k && (rc = jl_gemm_q6k_reserve(ctx, ctx->q6k_k > ctx->reserved_k ? ctx->reserved_k : ctx->q6k_k, ctx->reserved_tok))) return rc;
@@ -348,8 +353,10 @@ JL_EXPORT int jl_weight_upload_bank(jl_ctx *ctx, uint32_t type, const void *w_ho
     if (!ctx || !w_host || !out) return JL_EINVAL;
     std::lock_guard<std::mutex> lk(ctx->mu);
     JL_CUDA(ctx, cudaSetDevice(ctx->device));
+    jl_places_free(ctx, false);
     int rc = jl_grow_scratch(ctx, jl_gemv_scratch_bytes(type, k, type == JL_TYPE_Q8_0 ? 32 : 8));
     if (rc) return rc;
+    if (type == JL_TYPE_Q4_K && (rc = jl_xop_reserve(ctx, jl_gemv_scratch_bytes(type, k, 8)))) return rc;
     rc = jl_repack_upload(ctx, type, w_host, w_bytes, n_expert, nrows, k, out);
     if (rc == JL_OK && type == JL_TYPE_Q6_K) {     // the batch kernel's workspace, for as many tokens as were reserved
         if (k > ctx->q6k_k) ctx->q6k_k = k;

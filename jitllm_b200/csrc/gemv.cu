@@ -962,7 +962,14 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
                               "(jl_reserve sizes it)", ctx->scratch_cap, k, ntok, need);
         uint8_t *scratch = (uint8_t *)ctx->scratch;
         const bool prepared = x_dev == nullptr;   // the caller's kernels wrote the operand into the scratch already
-        const bool multi = q4k_use_multi(ctx, nrows, nsb, ntok, !prepared);
+        bool multi = q4k_use_multi(ctx, nrows, nsb, ntok, !prepared);
+        uint8_t *op = scratch;
+        if (multi && !prepared) {
+            // The form a small token count had before (wide, fused) reads x itself and shares nothing: this one converts x into
+            // a place that no other stream or graph writes to, or is not taken.
+            op = (uint8_t *)jl_operand_place(ctx, s, need);
+            if (!op) { multi = false; op = scratch; }
+        }
         const int idx = multi ? -1 : q4k_pick(ctx, nrows, nsb, ntok, !prepared);
         if (!multi && idx < 0) return jl_set_err(ctx, JL_DECLINED, "no decode variant fits %d x %d", nrows, k);
         cudaLaunchAttribute at[1];
@@ -974,7 +981,7 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((nsb + 3) / 4, ntok); cfg.blockDim = dim3(128); cfg.stream = s;
             cfg.attrs = at; cfg.numAttrs = nattr;
-            JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, q4k_xprep_kernel, x_dev, scratch, nsb, ntok));
+            JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, q4k_xprep_kernel, x_dev, op, nsb, ntok));
             ctx->st.launches++;
         }
         if (multi) {
@@ -987,7 +994,7 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((nrows + 16 * mrg - 1) / (16 * mrg)); cfg.blockDim = dim3((Q4KM_WPR * mrg + 1) * 32);
             cfg.dynamicSmemBytes = mf.smem; cfg.stream = s; cfg.attrs = at; cfg.numAttrs = nattr;
-            JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, mf.fn, w->map_sb16, expert * nrows, (const uint8_t *)scratch, out_dev, nrows, nsb,
+            JL_CUDA(ctx, cudaLaunchKernelEx(&cfg, mf.fn, w->map_sb16, expert * nrows, (const uint8_t *)op, out_dev, nrows, nsb,
                                             ctx->dev_status));
             ctx->st.launches++;
             return JL_OK;

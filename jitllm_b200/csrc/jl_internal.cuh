@@ -7,7 +7,9 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -89,6 +91,14 @@ struct jl_weight {
     uint32_t zc_flags;
 };
 
+// A graph's own memory for the calls that its capture took on one stream (workspace.cu).
+#define JL_XOP_SLOTS 8
+struct jl_place {
+    void *mem; size_t cap;
+    unsigned long long capture, stream;
+    std::shared_ptr<std::atomic<bool>> gone;     // set once nothing can replay the graph any more
+};
+
 struct jl_ctx {
     int device;
     jl_opts opts;
@@ -115,6 +125,9 @@ struct jl_ctx {
     void *x_dev; size_t x_cap;
     void *o_dev; size_t o_cap;
     void *scratch; size_t scratch_cap;
+    std::vector<jl_place> places;
+    // one slot per stream for the operand of a Q4_K call of 2..8 tokens (ids in order of arrival)
+    void *xop; size_t xop_slot; int xop_streams; unsigned long long xop_stream[JL_XOP_SLOTS];
     uint32_t multi_ready;               // forms of the 2..8-token decode kernel whose shared memory has been allowed
     // workspace of the Q6_K batch kernel, apart from the scratch (whose prepared operands outlive a call): sized for
     // what jl_reserve and the Q6_K uploads have asked for. q6k_done orders calls that come on another stream.
@@ -178,6 +191,10 @@ int jl_launch_gemv(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, 
 int jl_gemv_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, jl_choice *out);
 size_t jl_gemv_scratch_bytes(uint32_t type, int k, int ntok);
 int jl_grow_scratch(jl_ctx *ctx, size_t need);
+// workspace.cu -- where a call on `s` converts its activations; NULL: nowhere, and the call takes a kernel that does not
+void *jl_operand_place(jl_ctx *ctx, cudaStream_t s, size_t bytes);
+int jl_xop_reserve(jl_ctx *ctx, size_t bytes);
+void jl_places_free(jl_ctx *ctx, bool all);
 // ctx.cu: device copy of a host bank keyed on its address (as jl_matvec does for one matrix)
 int jl_resident_bank(jl_ctx *ctx, uint32_t type, const void *w, size_t w_bytes, int n_expert, int nrows, int k,
                      jl_weight **out);

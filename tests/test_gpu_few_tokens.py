@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from conftest import nmse, parity_err
-from jitllm_b200 import ACT_SILU, ACT_SWIGLU_OAI, MXFP4, Q4_K, Device, _lib, synth
+from jitllm_b200 import ACT_SILU, ACT_SWIGLU_OAI, MXFP4, Q4_K, Q8_0, Device, _lib, synth
 
 pytestmark = pytest.mark.gpu
 BAR = 2e-3
@@ -36,6 +36,76 @@ def test_q4k_tokens_inside_the_task(orc, nrows, k, ntok):
         assert np.isfinite(got).all() and nmse(got, ref) < 1e-8
         # the same integers per super-block as one token at a time; only the order of the f32 sums over super-blocks may differ
         assert parity_err(got, one.cpu().numpy()) <= (k / 256 + 4) * 2.0 ** -23
+
+
+def _few(d, rng, nrows=14336, k=4096, ntok=5, n=2):
+    """A shape that goes to the kernel with the tokens inside the task, n inputs and what each gives by itself."""
+    w = synth.q4k_matrix(rng, nrows, k)
+    d.Reserve(nrows, k, 32)
+    h = d.Upload(Q4_K, w, nrows, k)
+    xs = [torch.from_numpy(synth.activations(rng, ntok, k)).cuda() for _ in range(n)]
+    ref = [torch.empty(ntok, nrows, device="cuda") for _ in range(n)]
+    for x, r in zip(xs, ref):
+        d.MatMulDev(r, h, x, ntok, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return h, xs, ref
+
+
+def test_q4k_few_tokens_on_several_streams():
+    """Calls of one context on streams of their own do not meet: the same bits as alone for the first eight streams, the same
+    sums in another order beyond; a call of another format, whose operand lies in the context's scratch, runs beside them."""
+    rng = synth.rng_for(0xBA00)
+    ntok, n = 5, 10
+    with Device(0) as d:
+        h, xs, ref = _few(d, rng, n=n)
+        q8 = d.Upload(Q8_0, synth.matrix(rng, Q8_0, 4096, 4096), 4096, 4096)
+        x8, out8, want8 = torch.randn(32, 4096, device="cuda"), torch.empty(32, 4096, device="cuda"), torch.empty(32, 4096, device="cuda")
+        d.MatMulDev(want8, q8, x8, 32, torch.cuda.current_stream().cuda_stream)
+        outs = [torch.empty_like(ref[0]) for _ in range(n)]
+        ss, s8 = [torch.cuda.Stream() for _ in range(n)], torch.cuda.Stream()
+        torch.cuda.synchronize()
+        for _ in range(10):
+            d.MatMulDev(out8, q8, x8, 32, s8.cuda_stream)
+            for i in range(n):
+                d.MatMulDev(outs[i], h, xs[i], ntok, ss[i].cuda_stream)
+        torch.cuda.synchronize()
+        assert d.StatusPoll() and torch.equal(out8, want8)
+        for i in range(n):       # the default stream of `ref` holds a slot too
+            assert torch.equal(outs[i], ref[i]) if i < 7 else parity_err(outs[i].cpu().numpy(), ref[i].cpu().numpy()) <= (4096 / 256 + 4) * 2.0 ** -23
+
+
+def test_q4k_few_tokens_in_graphs_side_by_side():
+    """Two graphs of one context replayed on two streams beside a plain call on a third: each has its own operand; a graph's
+    place goes to the next one once it is gone, so that the hundredth still has one."""
+    rng = synth.rng_for(0xBA01)
+    ntok = 5
+    with Device(0) as d:
+        h, xs, ref = _few(d, rng, n=3)
+        outs = [torch.empty_like(r) for r in ref]
+        ss = [torch.cuda.Stream() for _ in range(3)]
+        graphs = []
+        for i in range(2):
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[i], stream=ss[i]):
+                for _ in range(4):
+                    d.MatMulDev(outs[i], h, xs[i], ntok, ss[i].cuda_stream)
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for i in range(2):
+                with torch.cuda.stream(ss[i]):
+                    graphs[i].replay()
+            d.MatMulDev(outs[2], h, xs[2], ntok, ss[2].cuda_stream)
+        torch.cuda.synchronize()
+        assert d.StatusPoll()
+        for o, r in zip(outs, ref):
+            assert torch.equal(o, r)
+        for i in range(100):
+            g = torch.cuda.CUDAGraph()
+            n0 = d.Stats().launches
+            with torch.cuda.graph(g, stream=ss[2]):
+                d.MatMulDev(outs[2], h, xs[2], ntok, ss[2].cuda_stream)
+            assert d.Stats().launches - n0 == 2          # the operand's launch and the matvec: not the one-launch form
+            g.reset()
 
 
 def _bank(dev, rng, E, H, F):
