@@ -332,9 +332,10 @@ void jl_weight_free(jl_ctx *ctx, jl_weight *w);
  * is gone), and a call without a place runs on a form that reads x itself. Such calls need no order among streams and graphs. */
 int jl_matvec_dev(jl_ctx *ctx, float *out_dev, const jl_weight *w, const float *x_dev, int ntok,
                   void *stream);
-/* Q6_K above 8 tokens keeps its converted activations in a workspace of the context (jl_reserve and the upload size it;
- * without it the row kernel runs): a call on another stream waits for the one before it. Parallel branches of ONE capture
- * over one context set JL_FLAG_DECODE_CONCURRENT, which keeps Q6_K on the row kernel. */
+/* Q6_K above 8 tokens keeps its converted activations in a workspace of the context, for the tokens that jl_reserve was told and
+ * the widest Q6_K matrix uploaded, whichever came first; a call that finds it too small runs on the row kernel. A call on another
+ * stream waits for the one before it; a captured call takes memory of its graph's own, as above, so that replays need no
+ * order against plain calls or other graphs. JL_FLAG_DECODE_CONCURRENT keeps Q6_K on the row kernel, which shares nothing. */
 int jl_matmul_dev(jl_ctx *ctx, void *out_dev, int out_dtype, const jl_weight *w, const void *x_dev,
                   int x_dtype, int ntok, void *stream);
 /* desc->gate/up/down are jl_weight* banks; biases and all other pointers are device pointers. */

@@ -59,10 +59,10 @@ JL_EXPORT int jl_open(int device, const jl_opts *opts, jl_ctx **out) {
     c->dev_status = nullptr;
     c->stat_pin = nullptr;
     c->moe_stage = nullptr; c->moe_stage_cap = 0;
-    c->q6k_work = nullptr; c->q6k_cap = 0; c->reserved_k = c->reserved_tok = c->q6k_k = 0;
+    c->q6k_work = nullptr; c->q6k_cap = 0; c->reserved_tok = c->q6k_k = 0;
     c->multi_ready = 0;
     c->xop = nullptr; c->xop_slot = 0; c->xop_streams = 0;
-    c->q6k_stream = nullptr; c->q6k_done = nullptr; c->q6k_recorded = c->q6k_captured = false;
+    c->q6k_stream = 0; c->q6k_done = nullptr; c->q6k_recorded = false;
     c->x_map = c->o_map = nullptr; c->x_map_cap = c->o_map_cap = 0; c->done_map = nullptr; c->done_seq = 0;
     const int words[4] = {0, (int)c->opts.wait_limit_us, 0, 0};   // code, wait limit, the done kernel's sequence counter, spare
     if (cudaMalloc(&c->dev_status, sizeof words) != cudaSuccess ||
@@ -97,7 +97,6 @@ JL_EXPORT void jl_close(jl_ctx *ctx) {
     if (ctx->xop) cudaFree(ctx->xop);
     jl_places_free(ctx, true);
     if (ctx->q6k_work) cudaFree(ctx->q6k_work);
-    for (void *p : ctx->q6k_outgrown) cudaFree(p);
     if (ctx->q6k_done) cudaEventDestroy(ctx->q6k_done);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->x_pin) cudaFreeHost(ctx->x_pin);
@@ -197,9 +196,8 @@ JL_EXPORT int jl_reserve(jl_ctx *ctx, int max_rows, int max_k, int max_tok) {
     int rc = jl_grow_scratch(ctx, need);
     if (rc) return rc;
     if ((rc = jl_xop_reserve(ctx, jl_gemv_scratch_bytes(JL_TYPE_Q4_K, k256, dtok)))) return rc;
-    if (k256 > ctx->reserved_k) ctx->reserved_k = k256;
     if (max_tok > ctx->reserved_tok) ctx->reserved_tok = max_tok;
-    if (ctx->q6k_k && (rc = jl_gemm_q6k_reserve(ctx, ctx->q6k_k > ctx->reserved_k ? ctx->reserved_k : ctx->q6k_k, ctx->reserved_tok))) return rc;
+    if (ctx->q6k_k && (rc = jl_gemm_q6k_reserve(ctx, ctx->q6k_k, ctx->reserved_tok))) return rc;
     return reserve_locked(ctx, (size_t)max_tok * max_k * 4, (size_t)max_tok * max_rows * 4);
 }
 
@@ -428,7 +426,11 @@ static int matmul_dev_locked(jl_ctx *ctx, void *out_dev, int out_dtype, const jl
             return jl_launch_gemm_tc5(ctx, out_dev, out_dtype, w, expert, x_dev, x_dtype, ntok, s);
         return jl_set_err(ctx, JL_DECLINED, "the decode kernels take f32 activations and outputs");
     }
-    if (ch.kernel == JL_K_TC5) return jl_launch_gemm_q6k(ctx, (float *)out_dev, w, expert, (const float *)x_dev, ntok, s);
+    if (ch.kernel == JL_K_TC5) {
+        rc = jl_launch_gemm_q6k(ctx, (float *)out_dev, w, expert, (const float *)x_dev, ntok, s);
+        if (rc != JL_DECLINED) return rc;
+        ch.kernel = JL_K_SIMT;
+    }
     return jl_launch_gemv(ctx, (float *)out_dev, w, expert, (const float *)x_dev, ntok, ch.kernel, s);
 }
 

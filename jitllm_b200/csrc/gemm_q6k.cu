@@ -392,12 +392,10 @@ size_t jl_gemm_q6k_scratch_bytes(int k, int ntok) {
 int jl_gemm_q6k_reserve(jl_ctx *ctx, int k, int ntok) {
     const size_t need = jl_gemm_q6k_scratch_bytes(k, ntok);
     if (ntok <= 8 || ctx->q6k_cap >= need) return JL_OK;
+    if (!ctx->q6k_done) JL_CUDA(ctx, cudaEventCreateWithFlags(&ctx->q6k_done, cudaEventDisableTiming));
     JL_CUDA(ctx, cudaDeviceSynchronize());   // an earlier launch may still read the old buffer
-    if (ctx->q6k_work) {
-        if (ctx->q6k_captured) ctx->q6k_outgrown.push_back(ctx->q6k_work);     // graphs replay with its address
-        else cudaFree(ctx->q6k_work);
-        ctx->q6k_work = nullptr; ctx->q6k_cap = 0; ctx->q6k_captured = false;
-    }
+    if (ctx->q6k_work) cudaFree(ctx->q6k_work);
+    ctx->q6k_work = nullptr; ctx->q6k_cap = 0;
     if (cudaMalloc(&ctx->q6k_work, need) != cudaSuccess) { cudaGetLastError(); ctx->q6k_work = nullptr; return JL_OK; }
     ctx->q6k_cap = need;
     return JL_OK;
@@ -438,28 +436,23 @@ static int q6g_launch(jl_ctx *ctx, const q6g_params &p, int tok_tiles, cudaStrea
     return JL_OK;
 }
 
+// JL_DECLINED: no workspace for this call, the row kernel takes it.
 int jl_launch_gemm_q6k(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expert, const float *x_dev, int ntok, cudaStream_t s) {
     const int nsb = w->k / 256, T = q6g_tile(ntok), tok_tiles = (ntok + T - 1) / T;
-    if (ctx->q6k_cap < jl_gemm_q6k_scratch_bytes(w->k, ntok))
-        return jl_set_err(ctx, JL_ENOMEM, "the Q6_K workspace holds %zu bytes, %d tokens x %d need %zu", ctx->q6k_cap, ntok, w->k,
-                          jl_gemm_q6k_scratch_bytes(w->k, ntok));
-    // One workspace per context. Calls on one stream follow each other; a call on another stream waits for the one before
-    // it. Inside a capture there is no event to wait for: a caller that captures parallel branches over one context says
-    // so with JL_FLAG_DECODE_CONCURRENT, which keeps Q6_K on the row kernel (no workspace).
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    JL_CUDA(ctx, cudaStreamIsCapturing(s, &cap));
-    if (cap != cudaStreamCaptureStatusNone) ctx->q6k_captured = true;
-    else {
-        if (!ctx->q6k_done) JL_CUDA(ctx, cudaEventCreateWithFlags(&ctx->q6k_done, cudaEventDisableTiming));
-        if (ctx->q6k_recorded && ctx->q6k_stream != s) JL_CUDA(ctx, cudaStreamWaitEvent(s, ctx->q6k_done, 0));
-    }
+    // Plain calls share the context's workspace: those of one stream follow each other, one on another stream waits for
+    // the call before it. A captured call works in memory of its graph's own, since nothing orders a replay against the rest.
+    const size_t need = jl_gemm_q6k_scratch_bytes(w->k, ntok);
+    jl_stream_state st;
+    if (!jl_stream_query(s, &st)) return JL_DECLINED;
+    uint8_t *planes = (uint8_t *)(st.graph ? jl_capture_place(ctx, st, need) : ctx->q6k_cap >= need ? ctx->q6k_work : nullptr);
+    if (!planes) return JL_DECLINED;
+    if (!st.graph && ctx->q6k_recorded && ctx->q6k_stream != st.stream) JL_CUDA(ctx, cudaStreamWaitEvent(s, ctx->q6k_done, 0));
     const size_t rows_off = (size_t)expert * w->nrows;
     q6g_params p;
     p.nrows = w->nrows; p.nsb = nsb; p.ntok = ntok; p.slices = q6g_slices(w->nrows, nsb, ntok, ctx->sm_count);
     p.w = w->data + rows_off * nsb * JL_Q6K_BLOCK;
     p.d = reinterpret_cast<const uint16_t *>(w->scales) + rows_off * nsb;
     p.x = x_dev; p.out = out_dev; p.status = ctx->dev_status;
-    uint8_t *planes = (uint8_t *)ctx->q6k_work;
     float *inv = (float *)(planes + (size_t)tok_tiles * T * w->k * 4);
     p.planes = planes; p.inv = inv;
     cudaLaunchConfig_t cfg = {};
@@ -480,9 +473,9 @@ int jl_launch_gemm_q6k(jl_ctx *ctx, float *out_dev, const jl_weight *w, int expe
     case 56: rc = q6g_launch<56>(ctx, p, tok_tiles, s); break;
     default: rc = q6g_launch<64>(ctx, p, tok_tiles, s); break;
     }
-    if (rc == JL_OK && cap == cudaStreamCaptureStatusNone) {
+    if (!st.graph) {          // also where the second launch was refused: the first one writes the planes
         JL_CUDA(ctx, cudaEventRecord(ctx->q6k_done, s));
-        ctx->q6k_stream = s;
+        ctx->q6k_stream = st.stream;
         ctx->q6k_recorded = true;
     }
     return rc;

@@ -130,12 +130,11 @@ struct jl_ctx {
     void *xop; size_t xop_slot; int xop_streams; unsigned long long xop_stream[JL_XOP_SLOTS];
     uint32_t multi_ready;               // forms of the 2..8-token decode kernel whose shared memory has been allowed
     // workspace of the Q6_K batch kernel, apart from the scratch (whose prepared operands outlive a call): sized for
-    // what jl_reserve and the Q6_K uploads have asked for. q6k_done orders calls that come on another stream.
+    // the widest Q6_K matrix uploaded and the tokens reserved. q6k_done orders plain calls that come on another stream;
+    // captured calls have a place of their own.
     void *q6k_work; size_t q6k_cap;
-    int reserved_k, reserved_tok, q6k_k;
-    cudaStream_t q6k_stream; cudaEvent_t q6k_done; bool q6k_recorded;
-    bool q6k_captured;                  // a capture has taken the workspace's address: an outgrown one is kept until jl_close
-    std::vector<void *> q6k_outgrown;
+    int reserved_tok, q6k_k;
+    unsigned long long q6k_stream; cudaEvent_t q6k_done; bool q6k_recorded;
     void *x_pin; size_t x_pin_cap;
     void *o_pin; size_t o_pin_cap;
     int *dev_status;        // device words: [0] code a kernel sets when a bounded wait ran out, [1] the limit (us)
@@ -192,6 +191,9 @@ int jl_gemv_choice(jl_ctx *ctx, uint32_t type, int nrows, int k, int ntok, jl_ch
 size_t jl_gemv_scratch_bytes(uint32_t type, int k, int ntok);
 int jl_grow_scratch(jl_ctx *ctx, size_t need);
 // workspace.cu -- where a call on `s` converts its activations; NULL: nowhere, and the call takes a kernel that does not
+struct jl_stream_state { cudaGraph_t graph; unsigned long long capture, stream; };   // graph: of the capture on the stream, or NULL
+bool jl_stream_query(cudaStream_t s, jl_stream_state *q);                               // false where the driver does not say
+void *jl_capture_place(jl_ctx *ctx, const jl_stream_state &st, size_t bytes);           // NULL: none
 void *jl_operand_place(jl_ctx *ctx, cudaStream_t s, size_t bytes);
 int jl_xop_reserve(jl_ctx *ctx, size_t bytes);
 void jl_places_free(jl_ctx *ctx, bool all);

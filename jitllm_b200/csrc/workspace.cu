@@ -17,27 +17,26 @@ static void CUDART_CB place_gone(void *flag) {
     delete f;
 }
 
-// The graph that a capture on `s` builds and its id, or NULL and the stream's id. False where the driver does not say.
-static bool stream_state(cudaStream_t s, unsigned long long *capture, cudaGraph_t *graph, unsigned long long *id) {
+bool jl_stream_query(cudaStream_t s, jl_stream_state *q) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    *graph = nullptr;
-    *id = (unsigned long long)(uintptr_t)s;
-    if (cudaStreamGetCaptureInfo(s, &st, capture, graph) != cudaSuccess) { cudaGetLastError(); return false; }
+    q->graph = nullptr;
+    q->stream = (unsigned long long)(uintptr_t)s;
+    if (cudaStreamGetCaptureInfo(s, &st, &q->capture, &q->graph) != cudaSuccess) { cudaGetLastError(); return false; }
     if (st == cudaStreamCaptureStatusActive) return true;
-    *graph = nullptr;
-    if (st != cudaStreamCaptureStatusNone || cudaStreamGetId(s, id) != cudaSuccess) { cudaGetLastError(); return false; }
+    q->graph = nullptr;
+    if (st != cudaStreamCaptureStatusNone || cudaStreamGetId(s, &q->stream) != cudaSuccess) { cudaGetLastError(); return false; }
     return true;
 }
 
-// `bytes` for the calls that capture `capture` takes on stream `id` (one after the other there): allocated at the first of
-// them, under the thread's relaxed capture mode, and given back once the graph, what was instantiated from it and its launches
-// are gone -- the runtime then drops the user object that the graph holds.
-static void *capture_place(jl_ctx *ctx, unsigned long long capture, cudaGraph_t graph, unsigned long long id, size_t bytes) {
+// `bytes` for the calls that a capture takes on one stream (one after the other there): allocated at the first of them, under
+// the thread's relaxed capture mode, and given back once the graph, what was instantiated from it and its launches are
+// gone -- the runtime then drops the user object that the graph holds.
+void *jl_capture_place(jl_ctx *ctx, const jl_stream_state &st, size_t bytes) {
     jl_place *free_place = nullptr;
     for (jl_place &p : ctx->places) {
         if (p.gone->load()) {
             if (p.cap >= bytes && (!free_place || p.cap < free_place->cap)) free_place = &p;
-        } else if (p.capture == capture && p.stream == id && p.cap >= bytes) {
+        } else if (p.capture == st.capture && p.stream == st.stream && p.cap >= bytes) {
             return p.mem;
         }
     }
@@ -63,12 +62,12 @@ static void *capture_place(jl_ctx *ctx, unsigned long long capture, cudaGraph_t 
         delete held;
         return nullptr;
     }
-    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    if (cudaGraphRetainUserObject(st.graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
         cudaGetLastError();
         cudaUserObjectRelease(obj, 1);
         return nullptr;
     }
-    free_place->capture = capture; free_place->stream = id; free_place->gone = flag;
+    free_place->capture = st.capture; free_place->stream = st.stream; free_place->gone = flag;
     return q.mem;
 }
 
@@ -99,14 +98,13 @@ int jl_xop_reserve(jl_ctx *ctx, size_t bytes) {
 
 void *jl_operand_place(jl_ctx *ctx, cudaStream_t s, size_t bytes) {
     if (s == ctx->stream) return ctx->scratch_cap >= bytes ? ctx->scratch : nullptr;
-    unsigned long long capture, id;
-    cudaGraph_t graph;
-    if (!stream_state(s, &capture, &graph, &id)) return nullptr;
-    if (graph) return capture_place(ctx, capture, graph, id, bytes);
+    jl_stream_state st;
+    if (!jl_stream_query(s, &st)) return nullptr;
+    if (st.graph) return jl_capture_place(ctx, st, bytes);
     if (ctx->xop_slot < bytes) return nullptr;
     int i = 0;
-    while (i < ctx->xop_streams && ctx->xop_stream[i] != id) i++;
+    while (i < ctx->xop_streams && ctx->xop_stream[i] != st.stream) i++;
     if (i == JL_XOP_SLOTS) return nullptr;
-    if (i == ctx->xop_streams) ctx->xop_stream[ctx->xop_streams++] = id;
+    if (i == ctx->xop_streams) ctx->xop_stream[ctx->xop_streams++] = st.stream;
     return (uint8_t *)ctx->xop + (size_t)i * ctx->xop_slot;
 }

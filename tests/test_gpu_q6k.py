@@ -76,6 +76,74 @@ def test_batch_kernel_in_a_graph_and_on_two_streams(orc):
         h.free()
 
 
+def test_batches_in_graphs_and_on_streams_side_by_side():
+    """Two graphs of one context and plain calls on two more streams, all with inputs of their own and no reserve in between, give
+    the bits that each gives alone; so do calls on streams that come and go, and a graph after its context's next reserve."""
+    rng = synth.rng_for(81)
+    nrows, k, ntok, n = 2048, 4096, 60, 4
+    w, xs = synth.matrix(rng, Q6_K, nrows, k), [torch.from_numpy(synth.activations(rng, ntok, k)).cuda() for _ in range(n)]
+    with Device(0) as dev:
+        dev.Reserve(nrows, k, ntok)
+        h = dev.Upload(Q6_K, w, nrows, k)
+        ref, outs = [torch.empty(ntok, nrows, device="cuda") for _ in range(n)], [torch.empty(ntok, nrows, device="cuda") for _ in range(n)]
+        for x, r in zip(xs, ref):
+            dev.MatMulDev(r, h, x, ntok, torch.cuda.current_stream().cuda_stream)
+        ss = [torch.cuda.Stream() for _ in range(n)]
+        torch.cuda.synchronize()
+        graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+        for i, g in enumerate(graphs):
+            n0 = dev.Stats().launches
+            with torch.cuda.graph(g, stream=ss[i]):
+                for _ in range(3):
+                    dev.MatMulDev(outs[i], h, xs[i], ntok, ss[i].cuda_stream)
+            assert dev.Stats().launches - n0 == 6                       # planes and GEMM, not the row kernel
+
+        def together():
+            for _ in range(10):
+                for i in range(2):
+                    with torch.cuda.stream(ss[i]):
+                        graphs[i].replay()
+                for i in (2, 3):
+                    dev.MatMulDev(outs[i], h, xs[i], ntok, ss[i].cuda_stream)
+            torch.cuda.synchronize()
+            assert dev.StatusPoll()
+            for o, r in zip(outs, ref):
+                assert torch.equal(o, r)
+                o.zero_()
+
+        together()
+        dev.Reserve(nrows, k, 3 * ntok)
+        together()
+        L = dev.lib
+        import ctypes as C
+        rt = C.CDLL("libcudart.so.12")
+        for i in range(40):                                             # a stream's handle may come back, its work is another's
+            s = C.c_void_p()
+            assert rt.cudaStreamCreateWithFlags(C.byref(s), 1) == 0
+            dev.MatMulDev(outs[i % n], h, xs[i % n], ntok, s.value)
+            assert rt.cudaStreamDestroy(s) == 0
+        torch.cuda.synchronize()
+        for o, r in zip(outs, ref):
+            assert torch.equal(o, r)
+        h.free()
+
+
+@pytest.mark.parametrize("first", ["upload", "reserve"])
+def test_workspace_for_the_widest_matrix_and_the_tokens_reserved(first):
+    """Whichever comes first, and whatever width the reserve names."""
+    nrows, k, ntok = 64, 1024, 40
+    w = synth.matrix(synth.rng_for(82), Q6_K, nrows, k)
+    with Device(0) as dev:
+        if first == "reserve":
+            dev.Reserve(nrows, 512, ntok)
+        h = dev.Upload(Q6_K, w, nrows, k)
+        if first == "upload":
+            assert dev.Select(Q6_K, nrows, k, ntok).kernel == K_SIMT
+            dev.Reserve(nrows, 512, ntok)
+        assert dev.Select(Q6_K, nrows, k, ntok).kernel == K_TC5
+        h.free()
+
+
 @pytest.mark.parametrize("dist", ["one_huge", "tiny", "huge", "zeros"])
 def test_batch_kernel_input_distributions(orc, dist):
     rng = synth.rng_for(78)
