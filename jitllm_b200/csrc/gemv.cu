@@ -774,17 +774,41 @@ static int q4k_find(int form, int warps, int stages, int rg, int minb, int nsb) 
     return -1;
 }
 
+// 2..8 tokens go through the kernel that keeps the tokens inside the task, unless the caller pinned a form or the warps, or
+// overlapped matvecs want one launch each. A trial or a measured verdict (of calls that hand x) names it by an index of its
+// own, behind the table's.
+static const int Q4K_MULTI_INDEX = Q4K_NVARIANTS;
+#define Q4K_FORM_MULTI 5       // its form in the verdict file
+static bool q4k_multi_fits(const jl_ctx *ctx, int ntok) {
+    const jl_opts &o = ctx->opts;
+    return ntok >= 2 && ntok <= 8 && o.decode_form == JL_FORM_AUTO && !o.pin_warps && !o.pin_stages && !o.pin_row_groups &&
+           !(o.flags & JL_FLAG_DECODE_CONCURRENT);
+}
+static bool q4k_use_multi(const jl_ctx *ctx, int nrows, int nsb, int ntok, bool have_x) {
+    if (!q4k_multi_fits(ctx, ntok)) return false;
+    if (ctx->force_variant >= 0) return ctx->force_variant == Q4K_MULTI_INDEX;
+    if (have_x) {
+        auto it = ctx->tuned.find(jl_tune_shape_key(JL_TYPE_Q4_K, nrows, nsb * 256, ntok));
+        if (it != ctx->tuned.end()) return it->second == Q4K_MULTI_INDEX;
+    }
+    // Small calls stay with a CTA per token: the tiles fetched again are few, and with x given their one launch (wide, fused)
+    // beats prep + multi. Measured, one call after the other: 9.4 against 12 us for 2..3 tokens of 4096 x 4096, 14.8 against 15.5
+    // for 5, 9.5 against 15 for 2 of 8192 x 2048, 17.0 against 17.2 for 2 of 4096 x 14336; 14.8 against 12.5 for 2 of 14336 x 4096,
+    // 20.0 against 15.6 for 8 of 4096 x 4096. With the operand prepared both are one launch: only the smallest stay.
+    return (long long)nrows * ntok > 8192 && (!have_x || (long long)nrows * ntok * nsb >= 400000);
+}
+
 // Which variant serves (nrows x nsb super-blocks, ntok tokens). have_x: the caller hands f32 activations (false:
 // the operand was already prepared by a producer kernel, so only the forms that read a prepared operand apply).
 // The reference decides per (quant, rows, k, ntok) (jit/gpu/tier/layer.go:10953-11016, tier.go:124-137).
 static int q4k_pick(const jl_ctx *ctx, int nrows, int nsb, int ntok, bool have_x) {
     const jl_opts &o = ctx->opts;
     const int nrg = (nrows + 15) / 16;
-    if (ctx->force_variant >= 0) return ctx->force_variant;       // a tuning trial is timing this variant
+    if (ctx->force_variant >= 0 && ctx->force_variant < Q4K_NVARIANTS) return ctx->force_variant;    // a tuning trial is timing this variant
     if (have_x && o.decode_form == JL_FORM_AUTO && !o.pin_warps && !(o.flags & JL_FLAG_DECODE_CONCURRENT)) {
         // a measured verdict for this shape (tune.cu) overrides the table below
         auto it = ctx->tuned.find(jl_tune_shape_key(JL_TYPE_Q4_K, nrows, nsb * 256, ntok));
-        if (it != ctx->tuned.end()) return it->second;
+        if (it != ctx->tuned.end() && it->second < Q4K_NVARIANTS) return it->second;
     }
     int form = o.decode_form;
     if (form < JL_FORM_AUTO || form > JL_FORM_L1) form = JL_FORM_AUTO;
@@ -827,20 +851,24 @@ int jl_gemv_tune_candidates(jl_ctx *ctx, int nrows, int k, int ntok, int *out, i
     int held = -1;
     auto it = ctx->tuned.find(key);
     if (it != ctx->tuned.end()) { held = it->second; ctx->tuned.erase(it); }
-    const int first = q4k_pick(ctx, nrows, nsb, ntok, true);
+    const int pick = q4k_pick(ctx, nrows, nsb, ntok, true);
+    const int first = pick >= 0 && q4k_use_multi(ctx, nrows, nsb, ntok, true) ? Q4K_MULTI_INDEX : pick;
     if (held >= 0) ctx->tuned[key] = held;
     if (first < 0) return 0;
     int n = 0;
     out[n++] = first;
     for (int i = 0; i < Q4K_NVARIANTS && n < cap; i++)
         if (i != first && q4k_variant_smem(q4k_variants[i], nsb) <= 200 * 1024) out[n++] = i;
+    if (first != Q4K_MULTI_INDEX && n < cap && q4k_multi_fits(ctx, ntok)) out[n++] = Q4K_MULTI_INDEX;
     return n;
 }
 int jl_gemv_variant_index(int form, int warps, int stages, int minb, int rg, int nsb) {
+    if (form == Q4K_FORM_MULTI) return warps == Q4KM_WPR && stages == 3 && minb == 1 && rg == 1 ? Q4K_MULTI_INDEX : -1;
     if (warps < 1 || stages < 1 || minb < 1 || rg < 1) return -1;
     return q4k_find(form, warps, stages, rg, minb, nsb);
 }
 void jl_gemv_variant_describe(int idx, int *form, int *warps, int *stages, int *minb, int *rg) {
+    if (idx == Q4K_MULTI_INDEX) { *form = Q4K_FORM_MULTI; *warps = Q4KM_WPR; *stages = 3; *minb = *rg = 1; return; }
     const q4k_variant &v = q4k_variants[idx];
     *form = v.form; *warps = v.warps; *stages = v.stages; *minb = v.minb; *rg = v.rg;
 }
@@ -848,21 +876,6 @@ void jl_gemv_variant_describe(int idx, int *form, int *warps, int *stages, int *
 static bool q4k_mma_ok(uint32_t type, int k) {
     // the activation operand of the whole row must fit one CTA's shared memory beside the default ring
     return type == JL_TYPE_Q4_K && k % 256 == 0 && q4k_find(JL_FORM_SPLIT, 0, 0, 0, 0, k / 256) >= 0;
-}
-
-// 2..8 tokens go through the kernel that keeps the tokens inside the task, unless the caller pinned a form or the warps, a
-// trial or a verdict names a variant, or overlapped matvecs want one launch each.
-static bool q4k_use_multi(const jl_ctx *ctx, int nrows, int nsb, int ntok, bool have_x) {
-    const jl_opts &o = ctx->opts;
-    if (ntok < 2 || ntok > 8 || ctx->force_variant >= 0 || o.decode_form != JL_FORM_AUTO || o.pin_warps || o.pin_stages || o.pin_row_groups ||
-        (o.flags & JL_FLAG_DECODE_CONCURRENT))
-        return false;
-    // Small calls stay with a CTA per token: the tiles fetched again are few, and with x given their one launch (wide, fused)
-    // beats prep + multi. Measured, one call after the other: 9.4 against 12 us for 2..3 tokens of 4096 x 4096, 14.8 against 15.5
-    // for 5, 9.5 against 15 for 2 of 8192 x 2048, 17.0 against 17.2 for 2 of 4096 x 14336; 14.8 against 12.5 for 2 of 14336 x 4096,
-    // 20.0 against 15.6 for 8 of 4096 x 4096. With the operand prepared both are one launch: only the smallest stay.
-    if ((long long)nrows * ntok <= 8192 || (have_x && (long long)nrows * ntok * nsb < 400000)) return false;
-    return !have_x || ctx->tuned.find(jl_tune_shape_key(JL_TYPE_Q4_K, nrows, nsb * 256, ntok)) == ctx->tuned.end();
 }
 
 static void q4k_fill_choice(const q4k_variant &v, int nrows, int nsb, int ntok, jl_choice *c) {

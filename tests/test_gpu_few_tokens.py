@@ -38,6 +38,31 @@ def test_q4k_tokens_inside_the_task(orc, nrows, k, ntok):
         assert parity_err(got, one.cpu().numpy()) <= (k / 256 + 4) * 2.0 ** -23
 
 
+def test_q4k_measured_selection_of_a_few_tokens(tmp_path):
+    """The duel has the kernel with the tokens inside the task among its candidates (31 us against 18 here, far outside the
+    margin), the verdict launches it, and a second context reads it from the file."""
+    nrows, k, ntok = 14336, 4096, 5
+    w = synth.q4k_matrix(synth.rng_for(0xBA02), nrows, k)
+    trials = []
+    for _ in range(2):
+        with Device(0) as d:
+            d.Reserve(nrows, k, ntok)
+            h = d.Upload(Q4_K, w, nrows, k)
+            before = d.Select(Q4_K, nrows, k, ntok)
+            d.WithTune(_lib.TUNE_ON, str(tmp_path))
+            ch = d.Tune(h, ntok)
+            trials.append(d.TuneStats()["trials"])
+            assert (ch.form, ch.warps, ch.grid) == (before.form, before.warps, before.grid) and ch.grid == -(-nrows // ch.rows_per_cta)
+            n0, out = d.Stats().launches, torch.empty(ntok, nrows, device="cuda")
+            d.MatMulDev(out, h, torch.randn(ntok, k, device="cuda"), ntok, torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            assert d.Stats().launches - n0 == ch.launches == 2
+            measured = d.TuneStats()["measured"]
+        if not measured and len(trials) == 1:
+            return                                     # a noisy box: every trial refused, the default stands (checked above)
+    assert trials[0] > 0 and trials[1] == 0
+
+
 def _few(d, rng, nrows=14336, k=4096, ntok=5, n=2):
     """A shape that goes to the kernel with the tokens inside the task, n inputs and what each gives by itself."""
     w = synth.q4k_matrix(rng, nrows, k)
