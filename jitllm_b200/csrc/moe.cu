@@ -712,8 +712,8 @@ static int moe_dev_locked(jl_ctx *ctx, float *out_dev, const void *h_dev, int h_
         return jl_set_err(ctx, JL_EINVAL, "jl_moe_desc.arm %d is not a known arm", d->arm);
     if (d->arm != JL_MOE_ARM_EXACT && (H > BS_MAX_KB * BS_KB || F > BS_MAX_KB * BS_KB))
         return jl_set_err(ctx, JL_DECLINED, "the block-scaled arm serves hidden and ffn up to %d", BS_MAX_KB * BS_KB);
-    if (d->arm == JL_MOE_ARM_EXACT &&
-        (wg->emin < 104 || wg->emax > 140 || wu->emin < 104 || wu->emax > 140 || wd->emin < 104 || wd->emax > 140))
+    const bool f16_scales = wg->emin >= 104 && wg->emax <= 140 && wu->emin >= 104 && wu->emax <= 140 && wd->emin >= 104 && wd->emax <= 140;
+    if (d->arm == JL_MOE_ARM_EXACT && !f16_scales)
         return jl_set_err(ctx, JL_DECLINED, "an MXFP4 block scale lies outside 2^-23..2^13, where f16 holds the weights exactly");
     const size_t need = jl_moe_scratch_bytes(ntok, E, K, H, F);
     if (ctx->scratch_cap < need)
@@ -740,9 +740,10 @@ static int moe_dev_locked(jl_ctx *ctx, float *out_dev, const void *h_dev, int h_
     at[0].val.programmaticStreamSerializationAllowed = 1;
     const int nattr = (ctx->opts.flags & JL_FLAG_NO_PDL) ? 0 : 1;
     auto cfg_of = [&](dim3 g, dim3 b) { cudaLaunchConfig_t c = {}; c.gridDim = g; c.blockDim = b; c.stream = s; c.attrs = at; c.numAttrs = nattr; return c; };
-    if (np <= (d->arm == JL_MOE_ARM_EXACT ? min(32, 2 * E) : 8) && d->arm != JL_MOE_ARM_BLOCK_SCALED) {
+    if (np <= (d->arm == JL_MOE_ARM_EXACT ? min(32, 2 * E) : 8) && d->arm != JL_MOE_ARM_BLOCK_SCALED && f16_scales) {
         // few pairs: matrix-vector products of the chosen experts (moe_dec.cuh says where the lines lie), the same or finer
-        // arithmetic than either arm
+        // arithmetic than either arm for these block scales; beyond them a block's sum times its scale can leave f32, which the
+        // block-scaled MMAs take
         moe_dec_params q = {};
         q.n_expert = E; q.top_k = K; q.hidden = H; q.ffn = F; q.act = d->act;
         q.cg = wg->data; q.cu = wu->data; q.cd = wd->data; q.eg = wg->scales; q.eu = wu->scales; q.ed = wd->scales;

@@ -164,3 +164,34 @@ def test_experts_over_routed_rows_with_each_parity_arm(dev, orc, arm):
     assert np.all(got[~live] == 123.0)                                   # skipped rows are not touched
     for w in (hg, hu, hd):
         w.free()
+
+
+@pytest.mark.parametrize("e", [3, 60, 104, 140, 200, 245])
+def test_parity_arm_takes_any_block_scale_at_any_batch(e):
+    """One row among two and among sixteen: the few-pair path serves only block scales that its f32 sums hold, so both give
+    the same layer (three-digit activations: the bar of the arm)."""
+    import ctypes as C
+
+    import torch
+    rng = synth.rng_for(0xBC00 + e)
+    E, H, F = 4, 128, 128
+    raw = [synth.mxfp4_matrix(rng, E * r, k) for r, k in ((F, H), (F, H), (H, F))]
+    for w, v in zip(raw, (120, e, 120)):
+        w.reshape(-1, 17)[:, 0] = v
+    st = torch.cuda.current_stream().cuda_stream
+    with Device(0) as dev:
+        dev.MoeReserve(16, E, 1, H, F)
+        banks = [dev.Upload(MXFP4, w, r, k, E) for w, (r, k) in zip(raw, ((F, H), (F, H), (H, F)))]
+        d = _lib.MoeDesc(struct_size=C.sizeof(_lib.MoeDesc), type=MXFP4, n_expert=E, top_k=1, hidden=H, ffn=F, act=0, norm=1, scale=1.0,
+                         gate=banks[0].handle, up=banks[1].handle, down=banks[2].handle, arm=_lib.MOE_ARM_BLOCK_SCALED_X3)
+        row = torch.from_numpy(synth.activations(rng, 1, H)).cuda() * 2.0 ** ((120 - e) // 3)     # the gated values stay within f32
+        outs = []
+        for n in (2, 16):
+            logits, out = torch.zeros(n, E, device="cuda"), torch.zeros(n, H, device="cuda")
+            logits[:, 1] = 5
+            sel, wt = torch.empty(n, 1, dtype=torch.int32, device="cuda"), torch.empty(n, 1, device="cuda")
+            dev.MoeDev(out, row.expand(n, H).contiguous(), logits, n, d, sel, wt, st)
+            outs.append(out[0].double())
+        torch.cuda.synchronize()
+        assert dev.StatusPoll() and bool(torch.isfinite(outs[1]).all())
+        assert float((outs[0] - outs[1]).norm() / outs[1].norm()) <= 2e-3
