@@ -646,8 +646,11 @@ JL_EXPORT int jl_aux_silu_mul_gemm(void *rows_f16, float *inv_scale, const float
     if (!rows_f16 || !inv_scale || !gu || n < 1 || ffn < 256 || ffn % 256) return JL_EINVAL;
     if (aux_misaligned(rows_f16) || aux_misaligned(gu)) return JL_EINVAL;
     if (ffn > 50 * 1024) return JL_DECLINED;      // the f32 row does not fit shared memory
+    // the attribute is the function's, not the call's: always its largest value, so that a call of another thread cannot lower it
+    // between this one's two steps
     const int smem = ffn * 4;
-    if (smem > 48 * 1024 - 64 && cudaFuncSetAttribute(aux_silu_mul_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+    if (smem > 48 * 1024 - 64 &&
+        cudaFuncSetAttribute(aux_silu_mul_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 50 * 1024 * 4) != cudaSuccess) {
         cudaGetLastError();
         return JL_ECUDA;
     }

@@ -50,6 +50,29 @@ def test_silu_mul_rounds_like_f32(ffn):
     assert float(((out.double() - ref).abs() / ref.abs()).max()) <= 3.6 * 2.0 ** -23
 
 
+def test_silu_mul_gemm_of_two_widths_from_two_threads():
+    """Both widths need more than 48 KB of shared memory; neither thread's setting may fail the other's launch."""
+    import threading
+    L, bad = _lib.load(), []
+
+    def loop(ffn):
+        s = torch.cuda.Stream()
+        gu = torch.zeros(1, 2 * ffn, device="cuda")
+        rows, inv = torch.empty(2, ffn, device="cuda", dtype=torch.float16), torch.empty(1, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(3000):
+            if L.jl_aux_silu_mul_gemm(rows.data_ptr(), inv.data_ptr(), gu.data_ptr(), 1, ffn, s.cuda_stream) != _lib.OK:
+                bad.append(ffn)
+        s.synchronize()
+
+    ts = [threading.Thread(target=loop, args=(ffn,)) for ffn in (51200, 12544)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
 @pytest.mark.parametrize("n,slots,hq,hkv,d,max_len", [(1, 1, 2, 1, 2, 1), (37, 3, 4, 2, 64, 40), (130, 2, 32, 8, 128, 130)])
 def test_rope_prefill_is_the_single_position_kernel_per_row(n, slots, hq, hkv, d, max_len):
     L = _lib.load()
