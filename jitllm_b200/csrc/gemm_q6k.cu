@@ -24,7 +24,8 @@
 // weight operands, 16 rows x 2 runs of 16 codes a warp, half a super-block (128 k) per stage.
 //
 // Activations that are not finite have no such integers: the prep kernel gives their super-block a NaN scale, the f32
-// accumulator becomes NaN, and the drain then computes that output as the row kernel does, element by element.
+// accumulator becomes NaN, and the drain then computes that output as both Q6_K kernels do, weight by weight (q6k_plain.cuh).
+#include "q6k_plain.cuh"
 #include "tc5.cuh"
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
@@ -114,25 +115,6 @@ __device__ __forceinline__ void q6g_mma(uint32_t d_tmem, uint64_t a_desc, uint64
 // Instruction descriptor, kind::i8: D s32, A and B signed, both K-major.
 __host__ __device__ constexpr uint32_t q6g_idesc(int m, int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-// The row kernel's sum over super-blocks [sb0, sb1) of one row and one token.
-__device__ __noinline__ float q6g_plain(const q6g_params &p, int row, int tok, int sb0, int sb1) {
-    float acc = 0.f;
-    for (int sb = sb0; sb < sb1; sb++) {
-        const size_t b = (size_t)row * p.nsb + sb;
-        const uint8_t *blk = p.w + b * JL_Q6K_BLOCK;
-        const float d = __half2float(__ushort_as_half(p.d[b]));
-        const float *x = p.x + ((size_t)tok * p.nsb + sb) * 256;
-        for (int e = 0; e < 256; e++) {
-            const int n = e >> 7, j = (e >> 5) & 3, l = e & 31;
-            const int byte = blk[n * 64 + l + (j & 1) * 32];
-            const int q = (j >= 2 ? byte >> 4 : byte & 0xF) | (((blk[128 + n * 32 + l] >> (2 * j)) & 3) << 4);
-            const int sc = (int)(int8_t)blk[192 + n * 8 + (l >> 4) + 2 * j];
-            acc = fmaf(__fmul_rn(__fmul_rn(d, (float)sc), (float)(q - 32)), x[e], acc);
-        }
-    }
-    return acc;
 }
 
 template <int T>
@@ -310,11 +292,10 @@ __global__ void __launch_bounds__(Q6G_THREADS, 1) gemm_q6k_kernel(const q6g_para
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + 8 * ab);
         }
-        // not finite: as the row kernel has it
 #pragma unroll
         for (int t = 0; t < T; t++)
             if (!(fabsf(acc[t]) < __int_as_float(0x7f800000)) && row < p.nrows && tt * T + t < p.ntok)
-                acc[t] = q6g_plain(p, row, tt * T + t, sb0, sb1);
+                acc[t] = q6k_plain(p.w + ((size_t)row * p.nsb + sb0) * JL_Q6K_BLOCK, drow, p.x + ((size_t)(tt * T + t) * p.nsb + sb0) * 256, nmine);
         if (p.slices == 1) {
 #pragma unroll
             for (int t = 0; t < T; t++)

@@ -20,6 +20,7 @@
 //                  and meet through shared memory in fixed order, so the result
 //                  is run-to-run bit-stable.
 #include "jl_internal.cuh"
+#include "q6k_plain.cuh"
 #include "tma.cuh"
 #include "raw_formats.cuh"
 
@@ -218,7 +219,11 @@ __global__ void __launch_bounds__(256) gemv_q6k_kernel(const uint8_t *__restrict
         float v = red[0][tid];
         for (int w = 1; w < (int)(blockDim.x >> 5); w++) v += red[w][tid];   // fixed order
         const int r = tid / NT, t = tid % NT;
-        if (row0 + r < nrows && tok0 + t < ntok) Y[(size_t)(tok0 + t) * nrows + row0 + r] = v;
+        if (row0 + r < nrows && tok0 + t < ntok) {
+            if (!(fabsf(v) < __int_as_float(0x7f800000)))
+                v = q6k_plain(data + (size_t)(row0 + r) * nsb * JL_Q6K_BLOCK, dplane + (size_t)(row0 + r) * nsb, X + (size_t)(tok0 + t) * k, nsb);
+            Y[(size_t)(tok0 + t) * nrows + row0 + r] = v;
+        }
     }
 }
 

@@ -186,3 +186,19 @@ def test_row_kernel_matches_float64(orc, nrows, k, ntok):
         got = run(dev, w, nrows, k, x)
     # 16 products, four runs per unit, k / 16384 units a thread, five shuffles, eight warps: under 64 roundings deep
     assert rel(got, ref) <= 64 * 2.0 ** -24 / 4
+
+
+@pytest.mark.parametrize("ntok", [1, 2, 5, 20])
+def test_activations_near_the_top_of_f32(orc, ntok):
+    """(q - 32) x overflows where the weight times x does not: such outputs are formed weight by weight, 1024 products one
+    after the other."""
+    rng = synth.rng_for(84 + ntok)
+    nrows, k = 70, 1024
+    w = synth.matrix(rng, Q6_K, nrows, k)
+    w.reshape(-1, 210)[:, 208:] = np.array([1e-5], np.float16).view(np.uint8)
+    x = (synth.activations(rng, ntok, k).clip(-3, 3) * np.float32(3e37)).astype(np.float32)
+    ref = orc.matmul_f64(Q6_K, w, x, nrows, k, ntok)
+    assert np.abs(ref).max() < 1e38 and np.abs(x).max() > np.finfo(np.float32).max / 32
+    with Device(0) as dev:
+        got = run(dev, w, nrows, k, x)
+    assert np.isfinite(got).all() and rel(got, ref) <= 1024 * 2.0 ** -24 / 4
