@@ -20,7 +20,6 @@
 //                  and meet through shared memory in fixed order, so the result
 //                  is run-to-run bit-stable.
 #include "jl_internal.cuh"
-#include "q6k_plain.cuh"
 #include "tma.cuh"
 #include "raw_formats.cuh"
 
@@ -124,8 +123,9 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const uint8_t *__restric
 // with them, loaded once for the R rows. A super-block is two halves of 128 elements; in a half, byte l of ql / ql + 32 /
 // qh carries elements l, l + 32, l + 64, l + 96 (low nibbles, low nibbles of the second run, high nibbles, high nibbles;
 // two bits of qh each), so 16 consecutive l are four runs of 16 consecutive elements, each with a scale of its own.
-// Codes become floats by byte placement (0x4B0000qq reads as 2^23 + q; minus (2^23 + 32) = q - 32, exact); a run's sum of
-// (q - 32) x is weighted by d * sc, which f32 holds exactly, so no weight is rounded at all. NT tokens share the codes.
+// Codes become floats by byte placement (0x468000qq reads as 2^14 + q 2^-9; minus (2^14 + 32 2^-9) = (q - 32) 2^-9, exact); a
+// run's sum of (q - 32) 2^-9 x is weighted by 2^9 d sc, which f32 holds exactly, so no weight is rounded at all, and 16 products of
+// any x that is finite sum without overflow. NT tokens share the codes.
 // Bound by what is in flight: a lane that read 2-byte words of the 210-byte blocks took 38.0 us for one token of 4096 x 14336;
 // the resident 208-byte blocks (see jl_weight) are read in 16-byte words, R x 58 bytes a thread at a time: 19.8 us, 2.4 TB/s.
 // R is 4 for every token count: the activations' loads (64 floats a unit and token) are then shared by four rows (with two, 4
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) gemv_q6k_kernel(const uint8_t *__restrict
             B[r] = ldg16(blk + n * 64 + 32 + 16 * j);
             H[r] = ldg16(blk + 128 + n * 32 + 16 * j);
             S[r] = __ldg(reinterpret_cast<const uint2 *>(blk + 192 + n * 8));
-            d[r] = half_bits_to_float(__ldg(dplane + b));
+            d[r] = half_bits_to_float(__ldg(dplane + b)) * 512.f;
         }
         const float *xu = X + (size_t)tok0 * k + (size_t)sb * 256 + n * 128 + j * 16;
 #pragma unroll
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) gemv_q6k_kernel(const uint8_t *__restrict
                     const uint32_t q4 = ((c < 2 ? l : l >> 4) & 0x0F0F0F0Fu) | (hb & 0x30303030u);
                     float w[4];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) w[e] = __uint_as_float(__byte_perm(q4, 0x4B000000u, 0x7650 + e)) - 8388640.f;
+                    for (int e = 0; e < 4; e++) w[e] = __uint_as_float(__byte_perm(q4, 0x46800000u, 0x7650 + e)) - 16384.0625f;
 #pragma unroll
                     for (int t = 0; t < NT; t++) {
                         q6k_fma2(g[r][t], make_float2(w[0], w[1]), make_float2(x[t].x, x[t].y));
@@ -219,11 +219,7 @@ __global__ void __launch_bounds__(256) gemv_q6k_kernel(const uint8_t *__restrict
         float v = red[0][tid];
         for (int w = 1; w < (int)(blockDim.x >> 5); w++) v += red[w][tid];   // fixed order
         const int r = tid / NT, t = tid % NT;
-        if (row0 + r < nrows && tok0 + t < ntok) {
-            if (!(fabsf(v) < __int_as_float(0x7f800000)))
-                v = q6k_plain(data + (size_t)(row0 + r) * nsb * JL_Q6K_BLOCK, dplane + (size_t)(row0 + r) * nsb, X + (size_t)(tok0 + t) * k, nsb);
-            Y[(size_t)(tok0 + t) * nrows + row0 + r] = v;
-        }
+        if (row0 + r < nrows && tok0 + t < ntok) Y[(size_t)(tok0 + t) * nrows + row0 + r] = v;
     }
 }
 

@@ -3,8 +3,8 @@
 #include "jl_internal.cuh"
 
 // The sum over `nsb` super-blocks of one row, each weight formed before it meets its activation, as quant.Dequant32 does
-// (format/quant/dequant.go:443-470). Both Q6_K kernels multiply codes by activations first and scale the sums: near the top of
-// f32 such a sum overflows where the output does not. They take an output that came out infinite or NaN from here.
+// (format/quant/dequant.go:443-470). The batch kernel multiplies codes by activations first and scales the sums: where an activation,
+// a scale or such a sum is not finite the output is formed here instead.
 // w: the row's resident blocks, d: their scales, x: the activations that go with them.
 static __device__ __noinline__ float q6k_plain(const uint8_t *w, const uint16_t *d, const float *x, int nsb) {
     float acc = 0.f;
