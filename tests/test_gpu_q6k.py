@@ -160,6 +160,39 @@ def test_batch_kernel_input_distributions(orc, dist):
     assert np.array_equal(got, ref) if dist == "zeros" else rel(got, ref) <= (4 + k / 256 / 2) * 2.0 ** -24
 
 
+# an element of every super-block F times the others and met by weights of zero; full and small scales; every group form
+@pytest.mark.parametrize("scales", [127, 16, 4])
+@pytest.mark.parametrize("F,ntok", [(1, 40), (30, 9), (100, 20), (150, 25), (400, 48), (1000, 64), (1e4, 50), (1e6, 70)])
+def test_batch_kernel_with_wide_super_blocks(orc, scales, F, ntok):
+    """The small elements alone make the sums: no further from float64 than an f32 chain of k FMAs, 2.1e-7 here as a random walk of
+    its roundings has it (2^-24 / sqrt 3 a step, the partial sums as large as sqrt(i / k) of the last: sqrt(k / 6) of them, half met)."""
+    rng = synth.rng_for(0xB900 + scales + ntok)
+    nrows, k = 256, 4096
+    w = synth.matrix(rng, Q6_K, nrows, k).copy()
+    b = w.reshape(-1, 210)
+    b[:, 192:208] = rng.integers(-scales, scales + 1, (b.shape[0], 16)).astype(np.int8).view(np.uint8)
+    b[:, 5] &= 0xF0                                                     # element 5: code 32, the weight 0
+    b[:, 128 + 5] = (b[:, 128 + 5] & 0xFC) | 2
+    x = rng.standard_normal((ntok, k)).astype(np.float32)
+    x[:, 5::256] = F
+    ref = orc.matmul_f64(Q6_K, w, x, nrows, k, ntok)
+    with Device(0) as dev:
+        got = run(dev, w, nrows, k, x)
+    print(f"scales {scales} F {F:g} {ntok} tokens: {rel(got, ref):.2e}")
+    assert rel(got, ref) <= 2.1e-7
+
+
+@pytest.mark.parametrize("scale", [1e-20, 1e-24, 1e-30, 1e-36])
+def test_batch_kernel_of_small_activations(orc, scale):
+    """Full precision down to the smallest rows (2^-80 and below are added as the row kernel does)."""
+    rng = synth.rng_for(86)
+    nrows, k, ntok = 64, 1024, 33
+    w, x = synth.matrix(rng, Q6_K, nrows, k), (synth.activations(rng, ntok, k) * np.float32(scale)).astype(np.float32)
+    with Device(0) as dev:
+        got = run(dev, w, nrows, k, x)
+    assert rel(got, orc.matmul_f64(Q6_K, w, x, nrows, k, ntok)) <= 12 * 2.0 ** -24
+
+
 def test_batch_kernel_not_finite():
     """Infinities and NaN give what the row kernel gives, in their own token only."""
     rng = synth.rng_for(79)
@@ -190,8 +223,8 @@ def test_row_kernel_matches_float64(orc, nrows, k, ntok):
 
 @pytest.mark.parametrize("ntok", [1, 2, 5, 20])
 def test_activations_near_the_top_of_f32(orc, ntok):
-    """(q - 32) x overflows where the weight times x does not: such outputs are formed weight by weight, 1024 products one
-    after the other."""
+    """32 x overflows where the weight times x does not: the row kernel's codes are scaled down, the batch kernel's integers know
+    no range. (1024 products one after the other at most.)"""
     rng = synth.rng_for(84 + ntok)
     nrows, k = 70, 1024
     w = synth.matrix(rng, Q6_K, nrows, k)
