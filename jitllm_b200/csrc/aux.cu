@@ -336,44 +336,46 @@ __device__ __forceinline__ void aux_mma_bf16(float (&d)[2], uint32_t a0, uint32_
 // and its own two-stage cp.async ring: no warp waits for another before the end of the CTA's positions. With one chunk to a
 // CTA (the small batches' form still) a batch of 64 at 2049 positions was 16,900 CTAs, each a load, five barriers, a
 // record, a fence and a ticket, and the cache came in at 3.9 TB/s; several chunks to a CTA keep the next tile on its way
-// while one is used and write a fraction of the records.
-#define ATT_STAGES 2
+// while one is used and write a fraction of the records. STAGES 1 is the form of one chunk to a CTA, where a second stage
+// would hold nothing: its tile alone, and four CTAs an SM instead of three (five and six spill). 2, 8, 13 sequences of 2049
+// positions: 14.4, 30.3, 44.5 us with the ring, 10.3, 24.3, 34.7 without.
 #define ATT_WARP_TILE (2 * 16 * ATT_ROW)              // 16 rows of K, 16 of V
-#define ATT_SMEM (4 * ATT_STAGES * ATT_WARP_TILE)
-template <int G>
-__global__ void __launch_bounds__(128, 3) aux_attn_decode_kernel(float *out, uint8_t *operand, const __nv_bfloat16 *q,
+#define ATT_SMEM(STAGES) (4 * (STAGES) * ATT_WARP_TILE)
+template <int G, int STAGES>
+__global__ void __launch_bounds__(128, STAGES == 1 ? 4 : 3) aux_attn_decode_kernel(float *out, uint8_t *operand, const __nv_bfloat16 *q,
                                                               const __nv_bfloat16 *k_cache, const __nv_bfloat16 *v_cache,
                                                               const long long *pos_dev, float *part, unsigned *tickets, int hkv,
                                                               int max_len, int nsplit, int per) {
     constexpr int HDR = (2 * G + 3) & ~3;              // max[G], sum[G], padded so that the V part is 16-byte aligned
     constexpr int STRIDE = HDR + G * ATT_D;
     extern __shared__ __align__(16) uint8_t tiles[];   // the warps' rings; the cross-warp sum red[4][G][128] reuses them
-    static_assert(4 * G * ATT_D * 4 <= ATT_SMEM, "reduction buffer must fit in the tiles");
+    static_assert(4 * G * ATT_D * 4 <= ATT_SMEM(STAGES), "reduction buffer must fit in the tiles");
     __shared__ float mred[4][G], lred[4][G];
     __shared__ unsigned last;
     const int split = blockIdx.x, kv = blockIdx.y, row = blockIdx.z, t = threadIdx.x, hq = hkv * G;
     AUX_PDL();
     long long len = *pos_dev + 1;
     if (len > max_len) len = max_len;
-    const int span = ATT_CHUNK * per, s0 = split * span;
+    const int span = STAGES == 1 ? ATT_CHUNK : ATT_CHUNK * per, s0 = split * span;
     const int cnt = len - s0 < 0 ? 0 : (len - s0 > span ? span : (int)(len - s0));
     float *my = part + (((size_t)row * hkv + kv) * nsplit + split) * STRIDE;
     if (cnt > 0) {
         const size_t base_row = ((size_t)row * hkv + kv) * max_len + s0;
+        const __nv_bfloat16 *kb = k_cache + base_row * ATT_D, *vb = v_cache + base_row * ATT_D;
         const int warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
         const int ntile = cnt > warp * 16 ? (cnt - warp * 16 + ATT_CHUNK - 1) / ATT_CHUNK : 0;
-        const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tiles) + warp * ATT_STAGES * ATT_WARP_TILE;
+        const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tiles) + warp * STAGES * ATT_WARP_TILE;
         // tile i of the warp: positions 64 i + 16 warp .. + 15, K rows then V rows; rows past cnt arrive as zeros
         auto issue = [&](int i) {
-            const uint32_t dst = ring + (i % ATT_STAGES) * ATT_WARP_TILE;
+            const uint32_t dst = ring + (i % STAGES) * ATT_WARP_TILE;
             const int p = i * ATT_CHUNK + warp * 16;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int piece = j * 32 + lane, r = piece >> 4, c = piece & 15;
-                const size_t at = (base_row + min(p + r, cnt - 1)) * ATT_D + c * 8;
+                const uint32_t at = (uint32_t)(min(p + r, cnt - 1) * ATT_D + c * 8);
                 const int bytes = p + r < cnt ? 16 : 0;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * ATT_ROW + c * 16), "l"(k_cache + at), "r"(bytes) : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (16 + r) * ATT_ROW + c * 16), "l"(v_cache + at), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * ATT_ROW + c * 16), "l"(kb + at), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (16 + r) * ATT_ROW + c * 16), "l"(vb + at), "r"(bytes) : "memory");
             }
         };
         if (ntile > 0) issue(0);
@@ -396,13 +398,16 @@ __global__ void __launch_bounds__(128, 3) aux_attn_decode_kernel(float *out, uin
 #pragma unroll
         for (int j = 0; j < 16; ++j) oacc[j][0] = oacc[j][1] = 0.f;
 #pragma unroll 1
-        for (int i = 0; i < ntile; ++i) {
-            __syncwarp();                                       // every lane is done with the stage that is refilled now
-            if (i + 1 < ntile) issue(i + 1);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        for (int i = 0; i < (STAGES == 1 ? 1 : ntile); ++i) {
+            if (STAGES == 1 && ntile == 0) break;
+            if (STAGES > 1) {
+                __syncwarp();                                   // every lane is done with the stage that is refilled now
+                if (i + 1 < ntile) issue(i + 1);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
             __syncwarp();
-            const uint32_t tile = ring + (i % ATT_STAGES) * ATT_WARP_TILE;
+            const uint32_t tile = ring + (i % STAGES) * ATT_WARP_TILE;
             const int p = i * ATT_CHUNK + warp * 16;
             // S[h][pos]: two n-tiles of 8 positions; lane (g, tq) ends up with S[g][p + 8 nt + 2 tq, + 1]
             float sv[4];
@@ -694,13 +699,13 @@ JL_EXPORT size_t jl_aux_attn_scratch_bytes(int n, int hq, int hkv, int max_len) 
 }
 
 template <typename... Args>
-static int aux_attn_launch(void (*kern)(Args...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess) { cudaGetLastError(); return JL_ECUDA; }
+static int aux_attn_launch(void (*kern)(Args...), int smem, dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return JL_ECUDA; }
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = ATT_SMEM; cfg.stream = s; cfg.attrs = at; cfg.numAttrs = 1;
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = at; cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, kern, args...) != cudaSuccess) { cudaGetLastError(); return JL_ECUDA; }
     return JL_OK;
 }
@@ -717,7 +722,12 @@ JL_EXPORT int jl_aux_attn_decode(float *out, void *operand_out, const void *q_bf
     // positions are nothing any more); one where the sequences alone do not fill the GPU, since there the CTAs' own time is
     // the call's.
     const int g = hq / hkv, chunks = (max_len + ATT_CHUNK - 1) / ATT_CHUNK;
-    const long long fill = (long long)n * hkv * chunks / (148 * 3 * 4);
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return JL_ECUDA;
+    }
+    const long long fill = (long long)n * hkv * chunks / (sms * 3 * 4);
     const int per = fill < 1 ? 1 : (fill > 8 ? 8 : (int)fill), nsplit = (chunks + per - 1) / per;
     if (operand_out && (g & 1)) return JL_EINVAL;      // a super-block of the operand is two heads
     unsigned *tickets = (unsigned *)scratch_zeroed_once;
@@ -727,11 +737,15 @@ JL_EXPORT int jl_aux_attn_decode(float *out, void *operand_out, const void *q_bf
     uint8_t *op = (uint8_t *)operand_out;
     const __nv_bfloat16 *q = (const __nv_bfloat16 *)q_bf16, *kc = (const __nv_bfloat16 *)k_cache_bf16,
                         *vc = (const __nv_bfloat16 *)v_cache_bf16;
+#define ATT_GO(G, ST) return aux_attn_launch(aux_attn_decode_kernel<G, ST>, ATT_SMEM(ST), grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per)
+#define ATT_CASE(G) case G: if (per == 1) ATT_GO(G, 1); ATT_GO(G, 2)
     switch (g) {
-    case 1: return aux_attn_launch(aux_attn_decode_kernel<1>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
-    case 2: return aux_attn_launch(aux_attn_decode_kernel<2>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
-    case 4: return aux_attn_launch(aux_attn_decode_kernel<4>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
-    case 8: return aux_attn_launch(aux_attn_decode_kernel<8>, grid, block, s, out, op, q, kc, vc, pos_dev, part, tickets, hkv, max_len, nsplit, per);
+    ATT_CASE(1);
+    ATT_CASE(2);
+    ATT_CASE(4);
+    ATT_CASE(8);
     }
+#undef ATT_CASE
+#undef ATT_GO
     return JL_ENOTSUP;
 }

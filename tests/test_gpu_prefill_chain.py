@@ -195,9 +195,10 @@ def test_wave_split_keeps_to_the_scratch():
     assert float((a - b).norm() / b.norm()) <= k / 16 * 2.0 ** -23
 
 
-# chunks per CTA from one to eight, a last CTA with part of its chunks, sequences that end in any chunk of it
+# chunks per CTA from one (the form without a ring) to eight, a cache far longer than its sequences, a last CTA with part of its chunks, sequences that end in any chunk of it
 @pytest.mark.parametrize("n,hq,hkv,pos,max_len", [(64, 32, 8, 2048, 2056), (64, 32, 8, 700, 2056), (64, 8, 8, 513, 1500), (33, 16, 8, 1000, 1001),
-                                                   (64, 64, 8, 15, 600), (20, 32, 8, 511, 512)])
+                                                   (64, 64, 8, 15, 600), (20, 32, 8, 511, 512), (13, 32, 8, 2048, 2056),
+                                                   (14, 32, 8, 2048, 2056), (13, 8, 8, 77, 130), (1, 32, 8, 700, 65536)])
 def test_attention_of_large_batches(n, hq, hkv, pos, max_len):
     L = _lib.load()
     d, g = 128, hq // hkv
