@@ -60,7 +60,7 @@ JL_EXPORT int jl_open(int device, const jl_opts *opts, jl_ctx **out) {
     c->stat_pin = nullptr;
     c->moe_stage = nullptr; c->moe_stage_cap = 0;
     c->q6k_work = nullptr; c->q6k_cap = 0; c->reserved_tok = c->q6k_k = 0;
-    c->multi_ready = 0;
+    c->multi_ready = c->q6k_ready = 0;
     c->xop = nullptr; c->xop_slot = 0; c->xop_streams = 0;
     c->q6k_stream = 0; c->q6k_done = nullptr; c->q6k_recorded = false;
     c->x_map = c->o_map = nullptr; c->x_map_cap = c->o_map_cap = 0; c->done_map = nullptr; c->done_seq = 0;

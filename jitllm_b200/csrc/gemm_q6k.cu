@@ -516,8 +516,8 @@ __global__ void __launch_bounds__(Q6G_THREADS, 1) gemm_q6k_kernel(const q6g_para
 
 // ------------------------------------------------------------------------- host
 
-// Tokens of a tile: the batch over the fewest tiles of 64 (8 T columns are all of TMEM there), rounded up to 8. The MMAs are
-// what bounds the kernel and their columns are 8 T: 203 tokens of 4096 x 14336 as four tiles of 64 took 154 us where tiles of 56 took 141, 140 tokens as
+// Tokens of a tile: the batch over the fewest tiles of 64 (8 T columns are all of TMEM there), rounded up to 8. Shared memory is
+// what bounds the kernel (82 % of its throughput on the SMs that work, the tensor pipe at 49 %), and the operands read from it grow with T: 203 tokens of 4096 x 14336 as four tiles of 64 took 154 us where tiles of 56 took 141, 140 tokens as
 // three of 64 153, of 48 124 (without the eighth digit product and the marks; now 146 and 142).
 static int q6g_tile(int ntok) {
     const int tiles = (ntok + 63) / 64, T = ((ntok + tiles - 1) / tiles + 7) & ~7;
@@ -573,7 +573,10 @@ static int q6g_launch(jl_ctx *ctx, const q6g_params &p, int tok_tiles, cudaStrea
     using L = q6g_smem<G0, G1>;
     static_assert(L::TOTAL <= 227 * 1024, "shared memory budget");
     static_assert(L::T * Q6G_RED_STRIDE * 4 <= L::BAR_OFS, "the partial tile reuses the stages");
-    JL_CUDA(ctx, cudaFuncSetAttribute(gemm_q6k_kernel<G0, G1>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+    if (!(ctx->q6k_ready >> (L::T / 8) & 1)) {       // once per context and form, not on every call
+        JL_CUDA(ctx, cudaFuncSetAttribute(gemm_q6k_kernel<G0, G1>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+        ctx->q6k_ready |= 1u << (L::T / 8);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.nrows + Q6G_ROWS - 1) / Q6G_ROWS * p.slices, tok_tiles); cfg.blockDim = dim3(Q6G_THREADS);
     cfg.dynamicSmemBytes = L::TOTAL; cfg.stream = s;

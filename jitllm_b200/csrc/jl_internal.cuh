@@ -128,6 +128,7 @@ struct jl_ctx {
     std::vector<jl_place> places;
     // one slot per stream for the operand of a Q4_K call of 2..8 tokens (ids in order of arrival)
     void *xop; size_t xop_slot; int xop_streams; unsigned long long xop_stream[JL_XOP_SLOTS];
+    uint32_t q6k_ready;                 // forms of the Q6_K batch kernel likewise (see multi_ready)
     uint32_t multi_ready;               // forms of the 2..8-token decode kernel whose shared memory has been allowed
     // workspace of the Q6_K batch kernel, apart from the scratch (whose prepared operands outlive a call): sized for
     // the widest Q6_K matrix uploaded and the tokens reserved. q6k_done orders plain calls that come on another stream;
