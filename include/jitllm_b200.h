@@ -165,8 +165,9 @@ int jl_stats_get(jl_ctx *ctx, jl_stats *out);
  * repack, bit-exactly), later calls reuse it. The caller guarantees the bytes
  * at w stay unchanged until jl_forget covers them. Types: Q4_K, Q8_0, MXFP4 on the tensor-core
  * decode kernels; Q4_0, Q5_0, Q5_1, Q5_K, Q6_K (what real Q4_K_M files mix in,
- * format/quant/dequant.go:85-146,399-470) on the one-warp-per-row kernel, which decodes each weight
- * exactly as quant.Dequant32 does (Q6_K batches above 8 tokens: the integer tensor cores, closer to exact still).
+ * format/quant/dequant.go:85-146,399-470) on row kernels: the first four decode each weight exactly as
+ * quant.Dequant32 does, Q6_K multiplies the codes and scales their sums, so that no weight is rounded (batches
+ * above 8 tokens on the integer tensor cores).
  * Any other type is DECLINED. */
 int jl_matvec(jl_ctx *ctx, float *out, uint32_t type, const void *w, size_t w_bytes,
               const float *x, int nrows, int k);

@@ -718,9 +718,11 @@ JL_EXPORT int jl_aux_attn_decode(float *out, void *operand_out, const void *q_bf
     if (aux_misaligned(out) || aux_misaligned(operand_out) || aux_misaligned(q_bf16) || aux_misaligned(k_cache_bf16) ||
         aux_misaligned(v_cache_bf16) || aux_misaligned(scratch_zeroed_once))
         return JL_EINVAL;
-    // Chunks per CTA: as many as leave four waves of three CTAs to an SM, eight at most (a record and a ticket every 512
-    // positions are nothing any more); one where the sequences alone do not fill the GPU, since there the CTAs' own time is
-    // the call's.
+    // Chunks per CTA: as many as leave four waves of three CTAs to an SM over the whole cache, eight at most (a record and a
+    // ticket every 512 positions are nothing any more); one where the cache does not fill the GPU, since there the CTAs' own
+    // time is the call's. The sequences' length is on the device and unknown here: in a cache much longer than they are, fewer CTAs work, but
+    // the idle ones cost more than that (one sequence of 2049 positions in 131,072: 38.9 us with a CTA per chunk, 22.6 with eight to a CTA; of 301
+    // 34.8 and 18.4; four of 301 in 32,768 36.9 and 20.5).
     const int g = hq / hkv, chunks = (max_len + ATT_CHUNK - 1) / ATT_CHUNK;
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {

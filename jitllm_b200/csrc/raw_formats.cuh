@@ -1,7 +1,8 @@
-// Element accessors of the ggml formats that stay as raw blocks on the device (Q4_0, Q5_0, Q5_1, Q5_K, Q6_K):
-// where element e of a block keeps its integer code, which scale fields go with it, and the weight's value computed
-// exactly as quant.Dequant32 computes it (format/quant/dequant.go:85-146, 399-470). Shared by the host unpack, the
-// resident unpack kernel and the one-warp-per-row matvec kernel, so all three read a block the same way.
+// Element accessors of the ggml formats without an integer tensor-core decode kernel: where element e of a block keeps its integer
+// code (Q4_0, Q5_0, Q5_1, Q5_K, and Q6_K, whose resident blocks are the raw ones without their d), which scale fields go
+// with it, and, for the first four, the weight's value computed exactly as quant.Dequant32 computes it
+// (format/quant/dequant.go:85-146, 399-441). Shared by the host unpack, the resident unpack kernel and the check kernel, so
+// all three read a block the same way.
 #pragma once
 #include <cstdint>
 

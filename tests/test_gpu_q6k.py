@@ -47,7 +47,8 @@ def test_batch_kernel_matches_float64(orc, nrows, k, ntok):
 
 
 def test_batch_kernel_in_a_graph_and_on_two_streams(orc):
-    """A captured call keeps its workspace when a later reserve outgrows it; calls on two streams share it in order."""
+    """A captured call has a workspace of its own, which a later reserve leaves alone; plain calls on two streams share the
+    context's in order."""
     rng = synth.rng_for(80)
     nrows, k, ntok = 256, 1024, 20
     w, xs = synth.matrix(rng, Q6_K, nrows, k), [torch.from_numpy(synth.activations(rng, ntok, k)).cuda() for _ in range(2)]
