@@ -910,6 +910,7 @@ __global__ void __launch_bounds__(BK_THREADS, 1) jl_block_kernel(const __grid_co
                     BK_FT(1);
                     const q4k_lane_tile w = q4k_lane_load(tiles + s * BK_TILE, g, t);
                     consumed++;
+                    fence_smem_reads();
                     __syncwarp();        // every lane holds its share: the stage may be refilled
                     if (fc.p < nphases) {
                         if (lane == 0) bk_fetch(fc, pinfo, maps, smem_u32(tiles + s * BK_TILE), smem_u32(bars + s));

@@ -481,6 +481,7 @@ gemv_q4k_tma_kernel(const __grid_constant__ CUtensorMap wmap, int row0, const vo
         const uint4 hB = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144);
         const uint4 qB0 = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144 + 16 + 32 * t);
         const uint4 qB1 = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144 + 32 + 32 * t);
+        fence_smem_reads();
         __syncwarp();  // every lane holds its share: the stage may be refilled
         if (lane == 0) {
             const int nx = sb + STAGES * WPR;
@@ -631,6 +632,7 @@ gemv_q4k_multi_kernel(const __grid_constant__ CUtensorMap wmap, int row0, const 
                 const uint4 qA1 = *reinterpret_cast<const uint4 *>(tile + g * 144 + 32 + 32 * t);
                 const uint4 qB0 = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144 + 16 + 32 * t);
                 const uint4 qB1 = *reinterpret_cast<const uint4 *>(tile + (g + 8) * 144 + 32 + 32 * t);
+                fence_smem_reads();
                 __syncwarp();  // every lane holds its share: the stage may be refilled
                 if (lane == 0) {
                     const int nx = sb + L::STAGES * Q4KM_WPR;

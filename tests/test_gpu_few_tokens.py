@@ -99,6 +99,33 @@ def test_q4k_few_tokens_on_several_streams():
             assert torch.equal(outs[i], ref[i]) if i < 7 else parity_err(outs[i].cpu().numpy(), ref[i].cpu().numpy()) <= (4096 / 256 + 4) * 2.0 ** -23
 
 
+def test_q4k_wide_form_with_the_gpu_full_of_other_calls():
+    """The form that converts x itself, on three of ten streams, gives the bits that it gives alone, every time: a tile's stage is
+    refilled only once its reads are done. (Without that order about one last call in seventeen had outputs of rows 8 to 15
+    of a tile wrong.)"""
+    rng = synth.rng_for(0xBA03)
+    ntok, n = 5, 10
+    with Device(0) as d, Device(0, decode_form=_lib.FORM_WIDE) as wide:
+        h, xs, _ = _few(d, rng, n=n)
+        hw, _, _ = _few(wide, synth.rng_for(0xBA03), n=1)
+        ref = [torch.empty(ntok, 14336, device="cuda") for _ in range(3)]
+        for i in range(3):
+            wide.MatMulDev(ref[i], hw, xs[7 + i], ntok, torch.cuda.current_stream().cuda_stream)
+        outs = [torch.empty_like(ref[0]) for _ in range(n)]
+        ss = [torch.cuda.Stream() for _ in range(n)]
+        torch.cuda.synchronize()
+        for _ in range(100):
+            for _ in range(10):
+                for i in range(7):
+                    d.MatMulDev(outs[i], h, xs[i], ntok, ss[i].cuda_stream)
+                for i in range(7, n):
+                    wide.MatMulDev(outs[i], hw, xs[i], ntok, ss[i].cuda_stream)
+            torch.cuda.synchronize()
+            for i in range(3):
+                assert torch.equal(outs[7 + i], ref[i])
+        assert d.StatusPoll() and wide.StatusPoll()
+
+
 def test_q4k_few_tokens_in_graphs_side_by_side():
     """Two graphs of one context replayed on two streams beside a plain call on a third: each has its own operand; a graph's
     place goes to the next one once it is gone, so that the hundredth still has one."""
