@@ -681,6 +681,7 @@ gemv_q4k_multi_kernel(const __grid_constant__ CUtensorMap wmap, int row0, const 
                     }
                 }
             }
+            if (it + L::XS < rounds) fence_smem_reads();     // the operand stage is refilled by a bulk copy
             __syncwarp();
             if (lane == 0) mbar_arrive(xempty + 8 * xs);
         }
