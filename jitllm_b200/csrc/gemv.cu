@@ -557,7 +557,7 @@ static size_t q4k_tma_smem(int warps, int stages, int nsb, bool fused = false, b
 // (640 B per super-block and token: 287 KB for 8 tokens of k = 14336) passes through a shared-memory ring of its own, four
 // super-blocks of all tokens a stage, filled by a warp that does nothing else; the four warps of a row group take one
 // super-block of a stage each. (Read from global memory through L1 instead, a task's loads came back one token after the
-// other: 22 us for that shape, and 61 against 42 for 8 tokens of 4096 x 14336; as it is 17.8 and 28.7, and a decode step of 8
+// other: 22 us for that shape, and 61 against 42 for 8 tokens of 4096 x 14336; as it is 17.8 (18.3 with the fences in front of refills) and 28.7, and a decode step of 8
 // sequences over two Llama-8B-wide blocks 287 us instead of 489.) RG row groups share the stage: two where the rows
 // fill the GPU with such CTAs (half the operand traffic), else one.
 #define Q4KM_WPR 4
